@@ -21,7 +21,12 @@
 // (one CTA per chunk and head) adds the partials in a fixed order and does the rest.  No atomics.
 #pragma once
 
-#include "seqmix.cuh"
+#include "gdn_fwd.cuh"
+
+constexpr int kGdnChunk = 64;
+constexpr int kGdnThreads = 256;
+using GdnDims = lewi::gdn::Dims;
+__device__ __forceinline__ float gdn_round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 constexpr int kGdnBwdVB = 32;          // state columns per CTA of kernel 1
 constexpr int kGdnBwdMaxDim = 128;     // head dimensions the register tiles are sized for (K, V <= 128)
@@ -156,11 +161,12 @@ __global__ void __launch_bounds__(kGdnThreads) gdn_bwd_scan_kernel(const __nv_bf
   // loads of one chunk: gcs and the decay factors, k (with its decay), w, u; optionally q (with its decay), attn, do
   auto load_chunk = [&](int n, bool backward) {
     const long long tok0 = (long long)n * C;
-    const uint8_t* cw = fws + (((long long)b * D.N + n) * D.H + h) * gdn_chunk_ws_bytes(K, V);
-    const __nv_bfloat16* u_in = reinterpret_cast<const __nv_bfloat16*>(cw);
-    const __nv_bfloat16* w_in = u_in + C * V;
-    const float* attn_in = reinterpret_cast<const float*>(w_in + C * K);
-    const float* gcs_in = attn_in + C * C;
+    const lewi::gdn::FwdWs FW = lewi::gdn::fwd_ws(D);
+    const long long fchunk = ((long long)b * D.N + n) * D.H + h;
+    const __nv_bfloat16* ut_in = reinterpret_cast<const __nv_bfloat16*>(fws + FW.ut) + fchunk * FW.v16 * 1024;
+    const __nv_bfloat16* w_in = reinterpret_cast<const __nv_bfloat16*>(fws + FW.w) + fchunk * C * K;
+    const __nv_bfloat16* attn_in = reinterpret_cast<const __nv_bfloat16*>(fws + FW.attn) + fchunk * 3 * C * C;
+    const float* gcs_in = reinterpret_cast<const float*>(fws + FW.gates) + fchunk * 3 * C;
     __syncthreads();   // the previous chunk is done with every buffer
     if (tid < C) {
       const float gc = gcs_in[tid], gl = gcs_in[C - 1];
@@ -196,14 +202,14 @@ __global__ void __launch_bounds__(kGdnThreads) gdn_bwd_scan_kernel(const __nv_bf
       const int r = i / VB, c = i - r * VB;
       const long long t = tok0 + r;
       const bool live = v0 + c < V;
-      sVn[r * VBP + c] = live ? __bfloat162float(u_in[r * V + v0 + c]) : 0.f;
+      sVn[r * VBP + c] = live ? __bfloat162float(ut_in[((v0 + c) / 16) * 1024 + ((((v0 + c) & 7) * 4 + ((r & 7) >> 1)) * 32) + (r >> 3) * 4 + (((v0 + c) >> 3) & 1) * 2 + (r & 1)]) : 0.f;
       if (backward)
         sDo[r * VBP + c] = (live && t < D.S) ? __bfloat162float(d_o[(((long long)b * D.S + t) * D.H + h) * V + v0 + c]) : 0.f;
     }
     if (backward) {
       for (int i = tid; i < C * C; i += kGdnThreads) {
         const int r = i / C, c = i - r * C;
-        sAt[r * (C + 1) + c] = attn_in[i];
+        sAt[r * (C + 1) + c] = c <= r ? (__bfloat162float(attn_in[i]) + __bfloat162float(attn_in[i + C * C])) + __bfloat162float(attn_in[i + 2 * C * C]) : 0.f;
       }
     }
     __syncthreads();
@@ -421,9 +427,9 @@ __global__ void __launch_bounds__(kGdnThreads, 1) gdn_bwd_chunk_kernel(const __n
   const GdnBwdWs W = gdn_bwd_ws(D);
   const long long chunks = (long long)D.B * D.N * D.H;
   const long long chunk = ((long long)b * D.N + n) * D.H + h;
-  const uint8_t* cw = fws + chunk * gdn_chunk_ws_bytes(K, V);
-  const float* attn_in = reinterpret_cast<const float*>(cw + (long long)C * V * 2 + (long long)C * K * 2);
-  const float* gcs_in = attn_in + C * C;
+  const lewi::gdn::FwdWs FW = lewi::gdn::fwd_ws(D);
+  const __nv_bfloat16* attn_in = reinterpret_cast<const __nv_bfloat16*>(fws + FW.attn) + chunk * 3 * C * C;
+  const float* gcs_in = reinterpret_cast<const float*>(fws + FW.gates) + chunk * 3 * C;
   const float* du_in = reinterpret_cast<const float*>(bws + W.du) + chunk * C * V;
   const float* pq = reinterpret_cast<const float*>(bws + W.pq) + chunk * C * K;
   const float* pk = reinterpret_cast<const float*>(bws + W.pk) + chunk * C * K;
@@ -518,13 +524,14 @@ __global__ void __launch_bounds__(kGdnThreads, 1) gdn_bwd_chunk_kernel(const __n
   for (int i4 = tid; i4 < C * C / 4; i4 += kGdnThreads) {
     const int r = i4 / (C / 4), c0 = (i4 - r * (C / 4)) * 4;
     const float4 da4 = psum4(pat, pstride_c, (long long)i4 * 4);
-    const float4 at4 = *reinterpret_cast<const float4*>(attn_in + i4 * 4);
+    float4 at4;
+    { float tt[4]; for (int x = 0; x < 4; ++x) tt[x] = (__bfloat162float(attn_in[i4 * 4 + x]) + __bfloat162float(attn_in[i4 * 4 + x + C * C])) + __bfloat162float(attn_in[i4 * 4 + x + 2 * C * C]); at4 = make_float4(tt[0], tt[1], tt[2], tt[3]); }
     const float da[4] = {da4.x, da4.y, da4.z, da4.w}, at[4] = {at4.x, at4.y, at4.z, at4.w};
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       const int c = c0 + x;
       const float d = c <= r ? da[x] : 0.f;
-      sX[r * CP + c] = d * at[x];
+      sX[r * CP + c] = c <= r ? d * at[x] : 0.f;
       sT[r * CP + c] = c <= r ? d * __expf(sG[r] - sG[c]) : 0.f;
     }
   }
