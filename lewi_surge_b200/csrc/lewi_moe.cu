@@ -8,8 +8,7 @@
 #include "router_gemm.cuh"
 #include "routing.cuh"
 #include "seqmix.cuh"
-#include "gdn_fwd.cuh"
-#include "seqmix_bwd.cuh"
+#include "gdn_bwd.cuh"
 
 #include <cstring>
 #include <mutex>
@@ -1206,8 +1205,7 @@ int lewi_gdn_chunk_fwd(void* stream, const void* q, const void* k, const void* v
 
 int64_t lewi_gdn_chunk_bwd_workspace_bytes(int B, int S, int H, int K, int V) {
   if (B <= 0 || S <= 0 || H <= 0 || K <= 0 || V <= 0) return LEWI_ERR_ARG;
-  GdnDims D{B, S, H, K, V, (S + kGdnChunk - 1) / kGdnChunk};
-  return gdn_bwd_ws(D).total;
+  return gdn::bwd_ws(gdn::Dims{B, S, H, K, V, (S + gdn::C - 1) / gdn::C}).total;
 }
 
 int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v, const float* g, const void* beta,
@@ -1217,39 +1215,21 @@ int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v
   if (!q || !k || !v || !g || !beta || !d_o || !fwd_workspace || !workspace || !dq || !dk || !dv || !dg || !dbeta)
     return LEWI_ERR_ARG;
   if (B <= 0 || S <= 0 || H <= 0 || K <= 0 || V <= 0) return LEWI_ERR_ARG;
-  if (K > kGdnBwdMaxDim || V > kGdnBwdMaxDim) return LEWI_ERR_LIMIT;
+  if (K > gdn::kMaxK || V > gdn::kMaxVBwd) return LEWI_ERR_LIMIT;
   if (K % 8 != 0 || V % 8 != 0) return LEWI_ERR_SHAPE;
+  if (!aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(fwd_workspace) || !aligned16(workspace) || !aligned16(dq) ||
+      !aligned16(dk) || !aligned16(dv))
+    return LEWI_ERR_SHAPE;
   if (fwd_workspace_bytes < lewi_gdn_chunk_workspace_bytes(B, S, H, K, V)) return LEWI_ERR_WORKSPACE;
   if (workspace_bytes < lewi_gdn_chunk_bwd_workspace_bytes(B, S, H, K, V)) return LEWI_ERR_WORKSPACE;
-  GdnDims D{B, S, H, K, V, (S + kGdnChunk - 1) / kGdnChunk};
-  const size_t smem_a = gdn_bwd_scan_smem_bytes(K), smem_b = gdn_bwd_chunk_smem_bytes(K, V);
-  if (smem_a > 220 * 1024 || smem_b > 220 * 1024) return LEWI_ERR_LIMIT;
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return LEWI_ERR_CUDA;
-  if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(gdn_bwd_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(gdn_bwd_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return LEWI_ERR_CUDA;
-    }
-    attr_set[dev] = true;
-  }
+  const gdn::Dims D{B, S, H, K, V, (S + gdn::C - 1) / gdn::C};
+  if ((long long)B * D.N * H > gdn::kMaxChunks || H > 65535 || B > 65535) return LEWI_ERR_LIMIT;
   cudaStream_t st = as_stream(stream);
-  const __nv_bfloat16* qb = reinterpret_cast<const __nv_bfloat16*>(q);
-  const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(k);
   const uint8_t* fws = reinterpret_cast<const uint8_t*>(fwd_workspace);
   uint8_t* bws = reinterpret_cast<uint8_t*>(workspace);
-  (void)g;   // the forward workspace holds the cumulative decay of every chunk
-  gdn_bwd_scan_kernel<<<dim3((unsigned)((V + kGdnBwdVB - 1) / kGdnBwdVB), (unsigned)H, (unsigned)B), kGdnThreads, smem_a, st>>>(
-      qb, kb, fws, h0, reinterpret_cast<const __nv_bfloat16*>(d_o), dh_final, bws, dh0, D);
-  LEWI_CHECK_LAUNCH();
-  gdn_bwd_chunk_kernel<<<dim3((unsigned)D.N, (unsigned)H, (unsigned)B), kGdnThreads, smem_b, st>>>(
-      qb, kb, reinterpret_cast<const __nv_bfloat16*>(v), reinterpret_cast<const __nv_bfloat16*>(beta), fws, bws,
-      reinterpret_cast<__nv_bfloat16*>(dq), reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv), dg,
-      reinterpret_cast<__nv_bfloat16*>(dbeta), D);
-  LEWI_CHECK_LAUNCH();
-  return LEWI_OK;
+  // the forward workspace holds q * scale and the cumulative decay of every chunk: q and g themselves are not read again
+  if (K <= 64) return gdn::backward<1>(st, k, v, beta, h0, d_o, dh_final, fws, bws, dq, dk, dv, dg, dbeta, dh0, D);
+  return gdn::backward<2>(st, k, v, beta, h0, d_o, dh_final, fws, bws, dq, dk, dv, dg, dbeta, dh0, D);
 }
 
 // ------------------------------------------------------------------------------------------------ whole layer
