@@ -265,6 +265,35 @@ __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles
   return t;
 }
 
+// prefix[e] = sum over x < e of count(rows of expert x), e in [0, E], by one warp: all offsets are requested at once and
+// scanned with shuffles.  (One thread that walked them took 8 us at 128 experts, before the first tile of every GEMM.)
+template <class F>
+__device__ __forceinline__ void expert_prefix(uint16_t* prefix, const int32_t* __restrict__ pad_offsets, int E, int lane, F count) {
+  constexpr int NV = 512 / 32;   // kMaxExperts / lanes
+  int lo[NV], hi[NV];
+#pragma unroll
+  for (int x = 0; x < NV; ++x) {
+    const int e = x * 32 + lane;
+    lo[x] = e < E ? pad_offsets[e] : 0;
+    hi[x] = e < E ? pad_offsets[e + 1] : 0;
+  }
+  int base = 0;
+#pragma unroll
+  for (int x = 0; x < NV; ++x) {
+    if (x * 32 >= E) break;
+    const int e = x * 32 + lane, c = e < E ? count(hi[x] - lo[x]) : 0;
+    int run = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += up;
+    }
+    if (e < E) prefix[e] = (uint16_t)(base + run - c);
+    base += __shfl_sync(0xffffffffu, run, 31);
+  }
+  if (lane == 0) prefix[E] = (uint16_t)min(base, 65535);
+}
+
 // 144 registers per thread: the register file is split over the SM's four schedulers (16,384 each), three of this
 // CTA's ten warps land on one scheduler, and 3 x 144 x 32 leaves it room for two 40-register warps of an exchange
 // CTA from another stream.  At the 168 the compiler would take by itself nothing else fits on the SM.  The
@@ -328,29 +357,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   }
   int n_units = 0;  // NN/NT: row blocks (or pairs of row blocks) to process
   if constexpr (MAJOR == TN) {
-    if (a.tn_part_rows > 0 && threadIdx.x == 32) {  // exclusive prefix of the experts' contraction-part counts
-      int run = 0;
-      for (int e = 0; e < a.E; ++e) {
-        pair_prefix[e] = (uint16_t)run;
-        const int rows_e = a.pad_offsets[e + 1] - a.pad_offsets[e];
-        run += max(1, (rows_e + a.tn_part_rows - 1) / a.tn_part_rows);
-      }
-      pair_prefix[a.E] = (uint16_t)min(run, 65535);
-    }
-  } else {
-    if constexpr (PAIR) {
-      if (a.pad_offsets != nullptr) {
-        if (threadIdx.x == 32) {  // exclusive prefix of ceil(blocks_e / 2); a few hundred adds at most
-          int run = 0;
-          for (int e = 0; e < a.E; ++e) {
-            pair_prefix[e] = (uint16_t)run;
-            const int nb = (a.pad_offsets[e + 1] - a.pad_offsets[e]) / BM;
-            run += (nb + 1) >> 1;
-          }
-          pair_prefix[a.E] = (uint16_t)min(run, 65535);
-        }
-      }
-    }
+    // exclusive prefix of the experts' contraction-part counts
+    if (a.tn_part_rows > 0 && warp == 1)
+      expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return max(1, (rows_e + a.tn_part_rows - 1) / a.tn_part_rows); });
+  } else if constexpr (PAIR) {
+    // exclusive prefix of ceil(blocks_e / 2)
+    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [](int rows_e) { return (rows_e / BM + 1) >> 1; });
   }
   if (warp == 1) {
     if constexpr (PAIR) {

@@ -37,6 +37,21 @@ def test_router_topk_bit_exact(cuda, t, e, k):
   check_tables(tb, logits, k, e)
 
 
+@pytest.mark.parametrize("t,e,k", [(128, 16, 6), (129, 16, 1), (2400, 8, 2), (127, 200, 3), (20000, 40, 4), (500, 512, 1)])
+def test_router_at_the_edges_of_its_two_paths(cuda, t, e, k):
+  """One CTA up to 128 tokens, chunks beyond; few experts (one partial sum per thread), an odd number, the most; and the
+  load-balance loss, a sum of e non-negative float32 terms: off by at most e * 2^-24 of it."""
+  from lewi_surge_b200 import layer
+  logits = np.random.default_rng(t + e).standard_normal((t, e)).astype(np.float32)
+  aux = torch.empty(1, dtype=torch.float32, device=cuda)
+  tb = layer.router_topk(to_dev(logits, torch.float32, cuda), k, aux_loss=aux)
+  L = check_tables(tb, logits, k, e)
+  p = np.exp(logits.astype(np.float64) - logits.max(1, keepdims=True))
+  p /= p.sum(1, keepdims=True)
+  want = e * float((L["counts"] / (t * k) * p.mean(0)).sum())
+  assert abs(float(aux.item()) - want) <= 1e-5 * want + e * 2.0 ** -24 * want
+
+
 def test_router_ties_pick_lower_index(cuda):
   from lewi_surge_b200 import layer
   rng = np.random.default_rng(5)
