@@ -19,6 +19,7 @@ constexpr int kRouteThreads = 512;
 constexpr int kRouteWarps = kRouteThreads / kWarp;
 constexpr int kFusedTokens = 128;       // one CTA routes up to this many tokens (two rounds of 16 warps x 4 tokens)
 constexpr int kMinChunkSlots = 128;     // lewi_route_workspace_bytes counts on it
+constexpr int kMaxChunkSlots = 32768;   // a chunk's expert ids and 17 rows of 512 counters fit in 200 KB of shared memory
 constexpr int kMaxExperts = 512;
 constexpr int kMaxTopK = 32;
 
@@ -697,16 +698,18 @@ __global__ void __launch_bounds__(256) split3_bf16_kernel(const float* __restric
 
 // ------------------------------------------------------------------------------------------------ host
 
-// Slots per chunk: one chunk per SM at most (see route_rank_kernel), whole tokens when fed logits (k slots each).
+// Slots per chunk: one chunk per SM (see route_rank_kernel) until a chunk no longer fits in shared memory, whole tokens when
+// fed logits (k slots each).
 inline int route_chunk_slots(long long M, int k, bool tokens) {
   const long long per = (M + num_sms() - 1) / num_sms();
   if (!tokens) {
     const long long s = (per + 255) / 256 * 256;
-    return (int)(s < 256 ? 256 : s);
+    return (int)(s < 256 ? 256 : (s > kMaxChunkSlots ? kMaxChunkSlots : s));
   }
   long long t = (per + k - 1) / k;                           // tokens: whole rounds of the CTA's 16 warps
   t = (t + kRouteWarps - 1) / kRouteWarps * kRouteWarps;
   if (t * k < kMinChunkSlots) t = (kMinChunkSlots + k - 1) / k;
+  if (t * k > kMaxChunkSlots) t = kMaxChunkSlots / k / kRouteWarps * kRouteWarps;
   return (int)(t * k);
 }
 

@@ -167,3 +167,14 @@ def test_group_tables(cuda):
   assert np.all(por[-3:] == -1)
   be = to_np(t["block_expert"])
   assert be[: pad[-1] // 128].tolist() == [0, 2, 3, 4, 5, 6, 7]
+
+
+def test_sort_of_more_slots_than_one_chunk_per_sm_holds(cuda):
+  """A chunk's expert ids live in shared memory: beyond one full chunk per SM there are more chunks, not a refusal."""
+  from lewi_surge_b200 import ops
+  m, e = 7_000_003, 500
+  idx = np.random.default_rng(8).integers(0, e, m).astype(np.int32)
+  order, pos = ops.sort_indices(to_dev(idx, torch.int32, cuda), e)
+  want = np.argsort(idx, kind="stable").astype(np.int32)
+  assert np.array_equal(to_np(order), want)
+  assert np.array_equal(to_np(pos)[want], np.arange(m, dtype=np.int32))
