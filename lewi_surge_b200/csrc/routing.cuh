@@ -51,7 +51,8 @@ __device__ __forceinline__ void warp_histogram(const int* s_e, int begin, int en
 template <int ER, int NT>
 __device__ __forceinline__ void warp_softmax_topk(const float* const (&rows)[NT], int E, int k, int lane,
                                                   int (&out_idx)[NT], float (&out_w)[NT], float (&p)[NT][ER]) {
-  uint32_t key[NT][ER];   // order-preserving image of the logits; 0: no such expert, or already chosen
+  // order-preserving image of the logits; 0: no such expert, or already chosen (the one NaN whose image is 0 takes 1)
+  uint32_t key[NT][ER];
   float mx[NT], sum[NT];
 #pragma unroll
   for (int i = 0; i < NT; ++i) {
@@ -61,7 +62,7 @@ __device__ __forceinline__ void warp_softmax_topk(const float* const (&rows)[NT]
       const int e = lane + r * kWarp;
       const bool in = e < E && rows[i] != nullptr;
       const float l = in ? rows[i][e] : 0.f;
-      key[i][r] = in ? float_order_key(l) : 0u;
+      key[i][r] = in ? max(float_order_key(l), 1u) : 0u;
       best = max(best, key[i][r]);
       p[i][r] = l;
     }

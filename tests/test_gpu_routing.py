@@ -178,3 +178,18 @@ def test_sort_of_more_slots_than_one_chunk_per_sm_holds(cuda):
   want = np.argsort(idx, kind="stable").astype(np.int32)
   assert np.array_equal(to_np(order), want)
   assert np.array_equal(to_np(pos)[want], np.arange(m, dtype=np.int32))
+
+
+@pytest.mark.parametrize("t", [64, 300])
+def test_router_keeps_a_nan_with_every_bit_set(cuda, t):
+  """0xFFFFFFFF (minus the NaN that the device makes) orders below every number, is still an expert, and shows in the weights."""
+  from lewi_surge_b200 import layer
+  logits = np.random.default_rng(t).standard_normal((t, 8)).astype(np.float32)
+  bits = logits.view(np.uint32)
+  bits[0] = 0xFFFFFFFF
+  bits[1, 2] = 0xFFFFFFFF
+  tb = layer.router_topk(torch.from_numpy(bits.view(np.int32)).to(cuda).view(torch.float32), 8)
+  idx, w = to_np(tb.topk_idx), to_np(tb.topk_w)
+  assert np.array_equal(idx[0], np.arange(8)) and idx[1, 7] == 2 and np.array_equal(np.sort(idx[1]), np.arange(8))
+  assert np.isnan(w[:2]).all() and np.isfinite(w[2:]).all()
+  assert np.array_equal(to_np(tb.counts), np.full(8, t))
