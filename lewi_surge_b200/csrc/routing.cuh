@@ -783,15 +783,15 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
     else { constexpr int ER = 16; rc_ = call; }               \
     if (rc_ != LEWI_OK) return rc_;          \
   } while (0)
+  const int chunk_slots = route_chunk_slots(M, k, logits != nullptr);
+  const int n_chunks = (int)((M + chunk_slots - 1) / chunk_slots);
+  const long long need = (long long)n_chunks * E * 8;
+  if (ws == nullptr || ws_bytes < need) return LEWI_ERR_WORKSPACE;   // also where the one-CTA path would not touch it
   if (logits != nullptr && T > 0 && T <= kFusedTokens) {
     const RouteFusedArgs fa{t, logits, topk_idx, topk_w, mpad, k};
     LEWI_ROUTE_ER(launch_route_fused<ER>(st, fa));
     return LEWI_OK;
   }
-  const int chunk_slots = route_chunk_slots(M, k, logits != nullptr);
-  const int n_chunks = (int)((M + chunk_slots - 1) / chunk_slots);
-  const long long need = (long long)n_chunks * E * 8;
-  if (ws == nullptr || ws_bytes < need) return LEWI_ERR_WORKSPACE;
   int32_t* chunk_hist = reinterpret_cast<int32_t*>(ws);
   float* chunk_probs = reinterpret_cast<float*>(chunk_hist + (long long)n_chunks * E);
   RouteChunkArgs ca;
