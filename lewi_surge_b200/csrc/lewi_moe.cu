@@ -1145,7 +1145,7 @@ int lewi_causal_conv1d_fwd(void* stream, const void* x, const void* w, void* y, 
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(y);
   cudaStream_t st = as_stream(stream);
-  LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<false, KT><<<grid, kConvThreads, 0, st>>>(xb, wb, yb, B, T, C)));
+  LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<KT><<<grid, kConvThreads, 0, st>>>(xb, wb, yb, B, T, C)));
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }
@@ -1160,23 +1160,26 @@ int lewi_causal_conv1d_bwd(void* stream, const void* x, const void* w, const voi
   const int runs = (T + kConvRun - 1) / kConvRun;
   if (dw != nullptr && (workspace == nullptr || workspace_bytes < (int64_t)B * runs * K * C * 4)) return LEWI_ERR_WORKSPACE;
   cudaStream_t st = as_stream(stream);
-  const dim3 grid((unsigned)((C / 8 + kConvThreads - 1) / kConvThreads), (unsigned)runs, (unsigned)B);
+  const int parts = (runs + kConvBwdRuns - 1) / kConvBwdRuns;   // per sequence; one fourth of what the workspace is sized for
+  const dim3 grid((unsigned)((C + kConvBwdChannels - 1) / kConvBwdChannels), (unsigned)parts, (unsigned)B);
   const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(w);
   const __nv_bfloat16* gb = reinterpret_cast<const __nv_bfloat16*>(g);
-  if (dx != nullptr) {
-    __nv_bfloat16* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
-    LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<true, KT><<<grid, kConvThreads, 0, st>>>(gb, wb, dxb, B, T, C)));
-    LEWI_CHECK_LAUNCH();
+  __nv_bfloat16* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
+  float* partial = reinterpret_cast<float*>(workspace);
+  if (dw == nullptr) {
+    LEWI_DISPATCH_TAPS(K, (causal_conv1d_bwd_kernel<KT, true, false><<<grid, kConvThreads, 0, st>>>(xb, wb, gb, dxb, nullptr, T, C)));
+  } else if (dx == nullptr) {
+    LEWI_DISPATCH_TAPS(K, (causal_conv1d_bwd_kernel<KT, false, true><<<grid, kConvThreads, 0, st>>>(xb, wb, gb, nullptr, partial, T, C)));
+  } else {
+    LEWI_DISPATCH_TAPS(K, (causal_conv1d_bwd_kernel<KT, true, true><<<grid, kConvThreads, 0, st>>>(xb, wb, gb, dxb, partial, T, C)));
   }
+  LEWI_CHECK_LAUNCH();
   if (dw != nullptr) {
-    float* partial = reinterpret_cast<float*>(workspace);
-    LEWI_DISPATCH_TAPS(K, (causal_conv1d_dw_kernel<KT><<<grid, kConvThreads, 0, st>>>(xb, gb, partial, B, T, C)));
-    LEWI_CHECK_LAUNCH();
     const int n = K * C;
-    conv_dw_reduce_kernel<<<(n + 255) / 256, 256, 0, st>>>(partial, B * runs, n,
-                                                          dw_dtype == LEWI_BF16 ? reinterpret_cast<__nv_bfloat16*>(dw) : nullptr,
-                                                          dw_dtype == LEWI_F32 ? reinterpret_cast<float*>(dw) : nullptr);
+    conv_dw_reduce_kernel<<<(n / 4 + kWarp - 1) / kWarp, 256, 0, st>>>(partial, B * parts, n,
+                                                                       dw_dtype == LEWI_BF16 ? reinterpret_cast<__nv_bfloat16*>(dw) : nullptr,
+                                                                       dw_dtype == LEWI_F32 ? reinterpret_cast<float*>(dw) : nullptr);
     LEWI_CHECK_LAUNCH();
   }
   return LEWI_OK;
