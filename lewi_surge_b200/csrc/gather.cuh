@@ -89,6 +89,9 @@ __global__ void __launch_bounds__(kGatherThreads) gather_rows_kernel(
 // (row_slot[r] < 0) become zero rows.  Every output row has exactly one writer, so this is the same function as
 // the row gather out[r] = x[row_slot[r] / k] -- but each source row is read once instead of k times at k distant
 // moments, which keeps the read side at T rows of DRAM traffic however large the source is against the L2.
+// A warp zeroes a few rows at a time: at decode sizes nearly all rows are such rows
+// (8 tokens over 128 experts: 6.1 MB of zeros; 13 us with 32 rows per warp, 7 us with 4).
+constexpr int kZeroRows = 4;
 template <int VPL>
 __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
     const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
@@ -123,9 +126,9 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
     }
   }
   // zero rows of the padded layout
-  for (long long r0 = warp0 * kWarp; r0 < rows; r0 += n_warps * kWarp) {
+  for (long long r0 = warp0 * kZeroRows; r0 < rows; r0 += n_warps * kZeroRows) {
     const long long r = r0 + lane;
-    const unsigned empty = __ballot_sync(0xffffffffu, r < rows && row_slot[r] < 0);
+    const unsigned empty = __ballot_sync(0xffffffffu, lane < kZeroRows && r < rows && row_slot[r] < 0);
     for (unsigned m = empty; m != 0; m &= m - 1) {
       const long long rr = r0 + (__ffs(m) - 1);
       for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + rr * d) + vi, make_uint4(0, 0, 0, 0));

@@ -252,7 +252,7 @@ int lewi_dispatch_rows(void* stream, const void* x, const int32_t* pos, const in
   const int vpl = pick_vpl(d, 2);
   if (vpl == 0) return LEWI_ERR_SHAPE;
   if (out_rows == 0) return LEWI_OK;
-  const int grid = gather_grid(T > out_rows / kWarp ? T : out_rows / kWarp + 1);
+  const int grid = gather_grid(T > out_rows / kZeroRows ? T : out_rows / kZeroRows + 1);
   cudaStream_t st = as_stream(stream);
   LEWI_DISPATCH_VPL(vpl, (dispatch_rows_kernel<VPL><<<grid, kGatherThreads, 0, st>>>(
                              reinterpret_cast<const __nv_bfloat16*>(x), pos, row_slot,
