@@ -28,22 +28,26 @@ constexpr int BK = 64;        // contraction elements per stage (128 bytes of bf
 constexpr int DATA_BYTES = 224 * 1024;         // operand ring + epilogue staging of one CTA
 constexpr int EPI_WARPS = 8;      // two warps per TMEM lane quarter, each takes half of the columns
 // Every epilogue warp moves its output (and the dSwiGLU epilogue also its g|u input) as TMA tiles of 32 rows x
-// 128 bytes (128-byte swizzle, 4 KB).  It owns two such tiles of staging, three under the SwiGLU epilogue, which
-// stores g, u and h of the same columns.  The operand ring gets the rest.
+// 128 bytes (128-byte swizzle, 4 KB).  It owns one such tile of staging, two where it needs g and u (or, scattering, a
+// second tile) at a time.  The operand ring gets the rest, since the main loop is bound by the loads in flight: with three tiles
+// under the SwiGLU epilogue (g, u and h at once) the ring had 4 stages per pair instead of 6, and the gate/up projection took
+// 412 us instead of 361 (196,608 rows over 128 x 512 experts, d = 1024), 311 instead of 261 (64 tokens, 256 x 768, d = 2048).
+// The plain epilogues (5 stages with two tiles) gained 0 to 5 %.
 constexpr int TILE_BYTES = 4096;
-__host__ __device__ constexpr int staging_per_warp(int epi) { return epi == 1 /* SWIGLU */ ? 3 * TILE_BYTES : 2 * TILE_BYTES; }
+__host__ __device__ constexpr int staging_tiles(int epi) { return epi == 2 /* DSWIGLU */ || epi == 4 /* SCATTER */ ? 2 : 1; }
+__host__ __device__ constexpr int staging_per_warp(int epi) { return staging_tiles(epi) * TILE_BYTES; }
 __host__ __device__ constexpr int ring_bytes(int epi) { return DATA_BYTES - EPI_WARPS * staging_per_warp(epi); }
 constexpr int A_BYTES = BM * BK * 2;           // 16 KB
 constexpr int CHUNK_BYTES = 64 * BK * 2;       // 8 KB: one [64 k][64 mn] box of an MN-major operand
-// One CTA per tile (cta_group::1): B is 256 x 64 = 32 KB, 3 stages of 48 KB (2 under the SwiGLU epilogue).
+// One CTA per tile (cta_group::1): B is 256 x 64 = 32 KB, 4 stages of 48 KB (3 where there are two staging tiles).
 // A CTA pair per 256-row tile (cta_group::2): each CTA holds its own 128 rows of A and HALF of B
-// (128 x 64 = 16 KB), 5 stages of 32 KB (4 under SwiGLU); the tensor cores of both SMs read both halves.
+// (128 x 64 = 16 KB), 6 stages of 32 KB (5 with two staging tiles); the tensor cores of both SMs read both halves.
 template <bool PAIR, int EPI = 0> struct Cfg {
   static constexpr int B_BYTES = PAIR ? BN * BK : BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = ring_bytes(EPI) / STAGE_BYTES;
 };
-constexpr int MAX_STAGES = 5;
+constexpr int MAX_STAGES = 6;
 constexpr int PAIR_PREFIX_BYTES = 1040;        // uint16 prefix per expert (E <= 512): row-block pairs (NN/NT) or contraction parts (TN)
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int TMEM_COLS = 512;
@@ -528,7 +532,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     uint8_t* stage = generic_base + RING_BYTES + (warp - 2) * staging_per_warp(EPI);
     uint32_t acc_it = 0;
     [[maybe_unused]] uint32_t epi_phase = 0;
-    [[maybe_unused]] TileStager<2> out2buf{stage, 0};
+    [[maybe_unused]] TileStager<staging_tiles(EPI)> out2buf{stage, 0};
     bool ok = true;
     for (int tile = tile_first; ok && tile < total_tiles; tile += tile_step) {
       const Tile t = decode_tile<MAJOR, EPI, PAIR>(a, tile, n_tiles_n, pair_prefix);
@@ -654,11 +658,29 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
         const int n64 = t.n0 + col_half * 64;
         if (rows_valid > 0 && n64 < n_end) {
           const float hsc = row_sc;
-          if (lane == 0) ptx::bulk_wait_read();   // the previous tile's three stores have read the staging tiles
-          __syncwarp();
-          uint8_t* buf_g = stage;
-          uint8_t* buf_u = stage + TILE_BYTES;
-          uint8_t* buf_h = stage + 2 * TILE_BYTES;
+          // g, then u, then h through the one staging tile (g and u are read from tensor memory twice)
+          if (a.out2 != nullptr) {
+#pragma unroll 1
+            for (int which = 0; which < 2; ++which) {
+              uint8_t* buf = out2buf.acquire(lane);
+#pragma unroll 1
+              for (int b = 0; b < 2; ++b) {
+                const int c = col_half * 2 + b;
+                if (t.n0 + c * 32 >= n_end) break;
+                uint32_t r[32];
+                float v[32];
+                if (has_acc) {
+                  ptx::tmem_ld_32x32(t_addr + which * (BN / 2) + c * 32, r);
+                  ptx::tmem_ld_wait();
+                }
+#pragma unroll
+                for (int q = 0; q < 32; ++q) v[q] = has_acc ? __uint_as_float(r[q]) : 0.f;
+                tile_put_bf16x32(buf, lane, b * 4, v);
+              }
+              out2buf.store3d(lane, &tm_d, buf, n64, which, (int)wrow0);
+            }
+          }
+          uint8_t* buf = out2buf.acquire(lane);
 #pragma unroll 1
           for (int b = 0; b < 2; ++b) {
             const int c = col_half * 2 + b;
@@ -668,31 +690,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
               ptx::tmem_ld_32x32(t_addr + c * 32, rg);
               ptx::tmem_ld_32x32(t_addr + BN / 2 + c * 32, ru);
               ptx::tmem_ld_wait();
+              if (b == 1 || t.n0 + (c + 1) * 32 >= n_end) release_acc();
             }
-            float g[32], u[32];
+            float g[32];
 #pragma unroll
             for (int q = 0; q < 32; ++q) {
-              g[q] = has_acc ? __uint_as_float(rg[q]) : 0.f;
-              u[q] = has_acc ? __uint_as_float(ru[q]) : 0.f;
+              const float gq = has_acc ? __uint_as_float(rg[q]) : 0.f, uq = has_acc ? __uint_as_float(ru[q]) : 0.f;
+              g[q] = gq * fast_sigmoid(gq) * uq * hsc;
             }
-            if (a.out2 != nullptr) {
-              tile_put_bf16x32(buf_g, lane, b * 4, g);
-              tile_put_bf16x32(buf_u, lane, b * 4, u);
-            }
-#pragma unroll
-            for (int q = 0; q < 32; ++q) g[q] = g[q] * fast_sigmoid(g[q]) * u[q] * hsc;
-            tile_put_bf16x32(buf_h, lane, b * 4, g);
+            tile_put_bf16x32(buf, lane, b * 4, g);
           }
-          ptx::fence_proxy_async();
-          __syncwarp();
-          if (lane == 0) {
-            if (a.out2 != nullptr) {
-              ptx::tma_store_3d(&tm_d, ptx::smem_u32(buf_g), n64, 0, (int)wrow0);
-              ptx::tma_store_3d(&tm_d, ptx::smem_u32(buf_u), n64, 1, (int)wrow0);
-            }
-            ptx::tma_store_2d(&tm_c, ptx::smem_u32(buf_h), n64, (int)wrow0);
-            ptx::bulk_commit();
-          }
+          out2buf.store2d(lane, &tm_c, buf, n64, (int)wrow0);
         }
       } else if constexpr (EPI == DSWIGLU) {
         const int f = a.N;
