@@ -272,12 +272,22 @@ int lewi_gather_reduce(void* stream, const void* y, const int32_t* pos, const fl
   const int vpl = pick_vpl(d, in_dtype == LEWI_BF16 ? 2 : 4);
   if (vpl == 0) return LEWI_ERR_SHAPE;
   if (n == 0) return LEWI_OK;
-  const int grid = gather_grid(n);
+  // one warp per 32 vectors where all of them are resident at once, else one per row
+  const int pieces = (int)(((long long)d * (in_dtype == LEWI_BF16 ? 2 : 4) / 16 + kWarp - 1) / kWarp);
+  const bool few = n * pieces <= (int64_t)num_sms() * (2048 / kWarp);
+  const int warps = kGatherThreads / kWarp;
+  const int grid = few ? (int)((n * pieces + warps - 1) / warps) : gather_grid(n);
   cudaStream_t st = as_stream(stream);
 #define LEWI_GR(TI, TO)                                                                                         \
-  LEWI_DISPATCH_VPL(vpl, (gather_reduce_kernel<TI, TO, VPL><<<grid, kGatherThreads, 0, st>>>(                   \
-                             reinterpret_cast<const TI*>(y), pos, w, reinterpret_cast<const TI*>(add0),         \
-                             reinterpret_cast<const TI*>(add1), reinterpret_cast<TO*>(out), n, k, d, n_y_rows)))
+  if (few) {                                                                                                    \
+    gather_reduce_few_kernel<TI, TO><<<grid, kGatherThreads, 0, st>>>(                                          \
+        reinterpret_cast<const TI*>(y), pos, w, reinterpret_cast<const TI*>(add0),                              \
+        reinterpret_cast<const TI*>(add1), reinterpret_cast<TO*>(out), n, k, d, pieces, n_y_rows);              \
+  } else {                                                                                                      \
+    LEWI_DISPATCH_VPL(vpl, (gather_reduce_kernel<TI, TO, VPL><<<grid, kGatherThreads, 0, st>>>(                 \
+                               reinterpret_cast<const TI*>(y), pos, w, reinterpret_cast<const TI*>(add0),       \
+                               reinterpret_cast<const TI*>(add1), reinterpret_cast<TO*>(out), n, k, d, n_y_rows))) \
+  }
   if (in_dtype == LEWI_BF16 && out_dtype == LEWI_BF16) { LEWI_GR(__nv_bfloat16, __nv_bfloat16); }
   else if (in_dtype == LEWI_BF16) { LEWI_GR(__nv_bfloat16, float); }
   else if (out_dtype == LEWI_BF16) { LEWI_GR(float, __nv_bfloat16); }

@@ -136,3 +136,22 @@ def test_dispatch_rows_equals_the_row_gather(cuda, t, e, k, d, skew):
   assert torch.equal(got, want)           # rows past the live blocks keep the fill value in both
   nb = int(tb.n_blocks.item()) * 128
   assert bool((got[nb:] == 7).all()) and nb <= tb.mpad
+
+
+@pytest.mark.parametrize("dtype,out", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.bfloat16, torch.float32),
+                                       (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("k", [1, 8, 9, 32])
+def test_gather_reduce_of_few_rows_gives_the_bits_of_many(cuda, dtype, out, k):
+  """A call of up to one resident wave of warps takes another kernel than a larger one: 1, 3 and 700 rows against the same rows
+  of a call of 10000, with weights, both addends, absent rows and a row length that fills no warp."""
+  from lewi_surge_b200 import ops
+  d, n, m = 264, 10000, 500
+  gen = torch.Generator(device=cuda).manual_seed(k)
+  y, a0, a1 = (torch.randn(r, d, generator=gen, device=cuda).to(dtype) for r in (m, n, n))
+  pos = torch.randint(-1, m, (n, k), generator=gen, device=cuda, dtype=torch.int32)
+  w = torch.rand(n, k, generator=gen, device=cuda)
+  many = ops.gather_reduce(y, pos, w, out, add0=a0, add1=a1)
+  bare = ops.gather_reduce(y, pos, None, out)
+  for r in (1, 3, 700):
+    assert torch.equal(ops.gather_reduce(y, pos[:r], w[:r], out, add0=a0[:r], add1=a1[:r]), many[:r])
+    assert torch.equal(ops.gather_reduce(y, pos[:r], None, out), bare[:r])
