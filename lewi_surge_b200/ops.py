@@ -332,7 +332,8 @@ class _RaggedDot(torch.autograd.Function):
     # dlhs = g . rhs[e]^T: rhs [E,K,N] read as the K-major operand with contraction over N
     dl_pad = grouped_gemm_nt(g_pad, b, block_expert, n_blocks, pad_offsets=pad_offsets)
     dlhs = gather_rows(dl_pad, padded_of_row)
-    drhs = grouped_gemm_tn(buf, g_pad, pad_offsets, ctx.e, out_dtype=torch.float32)
+    # rounded once from the float32 accumulators where the weights are bf16
+    drhs = grouped_gemm_tn(buf, g_pad, pad_offsets, ctx.e, out_dtype=torch.bfloat16 if ctx.rhs_dtype == torch.bfloat16 else torch.float32)
     return dlhs.to(ctx.lhs_dtype), drhs.to(ctx.rhs_dtype), None
 
 
