@@ -307,16 +307,17 @@ __device__ __forceinline__ void rev_scan(const CUtensorMap& tm_w, const CUtensor
 // Both scans of the backward pass: neither reads what the other writes.  CTAs below `nx` walk the sequence backwards, the others
 // forwards again.  A scan is a chain over the chunks, so running them side by side takes the longer one's time where the SMs
 // hold both (whole backward pass at K = V = 128: B=1, S=8192, H=4 587 -> 396 us; B=1, S=4096, H=8 373 -> 275 us; B=2, S=4096, H=8
-// 484 -> 442 us).  Where they do not, one launch each: mixed, B=8, S=4096, H=8 took 1564 us instead of 1488.
-template <int KB, int NG, int KS>
+// 485 -> 443 us).  Where they do not, one launch each: mixed, B=8, S=4096, H=8 took 1564 us instead of 1488.
+// SIDE: 0 the two by blockIdx, 1 the forward scan alone, 2 the reverse scan alone.
+template <int KB, int NG, int KS, int SIDE>
 __global__ void __launch_bounds__(scan_threads(NG * KS), 1)
 bwd_scans_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_at, const __grid_constant__ CUtensorMap tm_do, const ScanArgs fwd, const RevArgs rev,
                  int nx) {
-  if ((int)blockIdx.x < nx)
+  if (SIDE == 2 || (SIDE == 0 && (int)blockIdx.x < nx))
     rev_scan<KB, NG, KS>(tm_w, tm_q, tm_k, tm_at, tm_do, rev, blockIdx.x);
   else
-    fwd_scan<KB, NG, KS, true>(tm_w, tm_q, tm_k, tm_at, fwd, (int)blockIdx.x - nx);
+    fwd_scan<KB, NG, KS, true>(tm_w, tm_q, tm_k, tm_at, fwd, SIDE == 1 ? (int)blockIdx.x : (int)blockIdx.x - nx);
 }
 
 // ------------------------------------------------------------------------------------------------ chunk kernel
@@ -857,18 +858,25 @@ struct RevMaps {
   CUtensorMap w, q, k, at, d_o;
 };
 
+template <int KB, int NG, int KS, int SIDE>
+inline int launch_scans_side(cudaStream_t st, const RevMaps& m, const ScanArgs& fwd, const RevArgs& rev) {
+  static bool done[64] = {false};
+  constexpr int smem_f = ScanSmem<KB, NG, KS>::total, smem_r = RevSmem<KB, NG, KS>::total;
+  constexpr int smem = SIDE == 1 ? smem_f : (SIDE == 2 ? smem_r : (smem_r > smem_f ? smem_r : smem_f));
+  if (!allow_smem(bwd_scans_kernel<KB, NG, KS, SIDE>, smem, done)) return LEWI_ERR_CUDA;
+  const int nx = (rev.v16 + NG - 1) / NG;
+  bwd_scans_kernel<KB, NG, KS, SIDE><<<dim3((unsigned)(SIDE == 0 ? 2 * nx : nx), (unsigned)rev.D.H, (unsigned)rev.D.B), scan_threads(NG * KS), smem,
+                                       st>>>(m.w, m.q, m.k, m.at, m.d_o, fwd, rev, nx);
+  LEWI_CHECK_LAUNCH();
+  return LEWI_OK;
+}
 template <int KB, int NG, int KS>
 inline int launch_scans(cudaStream_t st, const RevMaps& m, const ScanArgs& fwd, const RevArgs& rev, bool together) {
-  static bool done[64] = {false};
-  constexpr int smem = RevSmem<KB, NG, KS>::total > ScanSmem<KB, NG, KS>::total ? RevSmem<KB, NG, KS>::total : ScanSmem<KB, NG, KS>::total;
-  if (!allow_smem(bwd_scans_kernel<KB, NG, KS>, smem, done)) return LEWI_ERR_CUDA;
-  const int nx = (rev.v16 + NG - 1) / NG;
-  for (int pass = together ? 1 : 0; pass < 2; ++pass) {   // one launch of both, or the forward scan (none in reverse) and then the other
-    bwd_scans_kernel<KB, NG, KS><<<dim3((unsigned)(together ? 2 * nx : nx), (unsigned)rev.D.H, (unsigned)rev.D.B), scan_threads(NG * KS), smem, st>>>(
-        m.w, m.q, m.k, m.at, m.d_o, fwd, rev, pass == 0 ? 0 : nx);
-    LEWI_CHECK_LAUNCH();
+  if constexpr (NG <= 2) {   // (four or eight groups are taken where twice as many CTAs do not fit)
+    if (together) return launch_scans_side<KB, NG, KS, 0>(st, m, fwd, rev);
   }
-  return LEWI_OK;
+  if (int rc = launch_scans_side<KB, NG, KS, 1>(st, m, fwd, rev)) return rc;
+  return launch_scans_side<KB, NG, KS, 2>(st, m, fwd, rev);
 }
 
 template <int KB, int VB>
