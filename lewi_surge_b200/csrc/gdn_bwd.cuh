@@ -77,7 +77,7 @@ struct RevArgs {
 // The forward scan's structure with dh^T in the registers and the chunks in reverse:
 //   dv^T = (dh^T k^T) exp(gcs_last - gcs) + do^T attn;   dh^T <- dh^T exp(gcs_last) + (do exp(gcs))^T q - dv^T w.
 // Token pairs (16 tokens) are kept in the warp's own order throughout, the OP pairs that it finishes first.
-// 636 m16n8k16 per group and chunk at K = 128.  B=8, S=4096, H=8, K=V=128: 0.28 ms, the forward pass before it 0.19 ms (both
+// 636 m16n8k16 per group and chunk at K = 128.  B=8, S=4096, H=8, K=V=128: 0.31 ms, the forward pass before it 0.20 ms (both
 // together 6.7 ms in float32 on the CUDA cores).
 template <int KB, int NG, int KS>
 __device__ __forceinline__ void rev_scan(const CUtensorMap& tm_w, const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_at,
@@ -206,8 +206,8 @@ __device__ __forceinline__ void rev_scan(const CUtensorMap& tm_w, const CUtensor
       for (int i = 0; i < OP; ++i) {
         const int p = pair_at(i);
         if (p > ks) continue;
-#pragma unroll
-        for (int w3 = 2; w3 >= 0; --w3) mma2(dv[2 * i], dv[2 * i + 1], da.r, ld_b_t(st + St::at + w3 * kBox, ks * 16, p, L));
+        const Frag4 b[3] = {ld_b_t(st + St::at, ks * 16, p, L), ld_b_t(st + St::at + kBox, ks * 16, p, L), ld_b_t(st + St::at + 2 * kBox, ks * 16, p, L)};
+        mma2_x3(dv[2 * i], dv[2 * i + 1], da.r, b);
       }
     }
     if constexpr (KS > 1) {
@@ -219,33 +219,28 @@ __device__ __forceinline__ void rev_scan(const CUtensorMap& tm_w, const CUtensor
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(v_bar);
     }
+    // dh = dh exp(gcs_last) + (do exp(gcs))^T q, while the other warps' parts of dv arrive
     const float dec = gates[2 * C - 1];
-#pragma unroll
-    for (int t = 0; t < 2 * KT; ++t)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) dh[t][e] *= dec;
-    // dh += (do exp(gcs))^T q, while the other warps' parts of dv arrive
+    constexpr int CW = KT >= 2 ? 2 : 1;   // column pairs side by side
+    Frag3x4 af[4];
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       const Frag4 da = ld_a_t(st + St::d_o, ks * 16, dp, L);
       const float2 e0 = *reinterpret_cast<const float2*>(gates + C + ks * 16 + kc), e1 = *reinterpret_cast<const float2*>(gates + C + ks * 16 + 8 + kc);
-      Frag3x4 ef;
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const float2 e = x < 2 ? e0 : e1;
-        split3(bf16_lo(da.r[x]) * e.x, bf16_hi(da.r[x]) * e.y, ef.p[0][x], ef.p[1][x], ef.p[2][x]);
+        split3(bf16_lo(da.r[x]) * e.x, bf16_hi(da.r[x]) * e.y, af[ks].p[0][x], af[ks].p[1][x], af[ks].p[2][x]);
       }
-      constexpr int CW = KT >= 2 ? 2 : 1;
+    }
 #pragma unroll
-      for (int cp = 0; cp < KT; cp += CW) {
-        Frag4 qf[CW];
+    for (int cp = 0; cp < KT; cp += CW) {
+      float add[2 * CW][4];
+      chunk_sum<CW>(add, af, [&](int ks, int x) { return ld_b_t(st + St::q, ks * 16, kq * KT + cp + x, L); });
 #pragma unroll
-        for (int x = 0; x < CW; ++x) qf[x] = ld_b_t(st + St::q, ks * 16, kq * KT + cp + x, L);
+      for (int t = 0; t < 2 * CW; ++t)
 #pragma unroll
-        for (int w3 = 2; w3 >= 0; --w3)
-#pragma unroll
-          for (int x = 0; x < CW; ++x) mma2(dh[2 * (cp + x)], dh[2 * (cp + x) + 1], ef.p[w3], qf[x]);
-      }
+        for (int e = 0; e < 4; ++e) dh[2 * cp + t][e] = fmaf(dh[2 * cp + t][e], dec, add[t][e]);
     }
     if constexpr (KS > 1) {
       ok = ptx::mbar_wait(v_bar, it & 1u, abort_flag);
@@ -269,25 +264,15 @@ __device__ __forceinline__ void rev_scan(const CUtensorMap& tm_w, const CUtensor
     for (int t = 0; t < OWN; ++t) dv_out[(2 * pair_at(t >> 1) + (t & 1)) * 32] = make_float4(dv[t][0], dv[t][1], dv[t][2], dv[t][3]);
     // dh -= dv^T w
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 4; ++i) split_acc(dv[2 * i], dv[2 * i + 1], af[i]);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        dv[2 * i][e] = -dv[2 * i][e];
-        dv[2 * i + 1][e] = -dv[2 * i + 1][e];
-      }
-      Frag3x4 vf;
-      split_acc(dv[2 * i], dv[2 * i + 1], vf);
-      constexpr int CW = KT >= 2 ? 2 : 1;
+    for (int cp = 0; cp < KT; cp += CW) {
+      float sub[2 * CW][4];
+      chunk_sum<CW>(sub, af, [&](int i, int x) { return ld_b_t(st + St::w, pair_at(i) * 16, kq * KT + cp + x, L); });
 #pragma unroll
-      for (int cp = 0; cp < KT; cp += CW) {
-        Frag4 wf[CW];
+      for (int t = 0; t < 2 * CW; ++t)
 #pragma unroll
-        for (int x = 0; x < CW; ++x) wf[x] = ld_b_t(st + St::w, pair_at(i) * 16, kq * KT + cp + x, L);
-#pragma unroll
-        for (int w3 = 2; w3 >= 0; --w3)
-#pragma unroll
-          for (int x = 0; x < CW; ++x) mma2(dh[2 * (cp + x)], dh[2 * (cp + x) + 1], vf.p[w3], wf[x]);
-      }
+        for (int e = 0; e < 4; ++e) dh[2 * cp + t][e] -= sub[t][e];
     }
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(empty_bar(s));
@@ -384,7 +369,10 @@ __device__ __forceinline__ float quad_sum(float v) {
 // One CTA of 16 warps per chunk and head.  [64, K] results: warp (wm, wc) owns 16 tokens and a quarter of the columns;
 // [64, 64] results: one 16 x 16 tile.  What contracts over V (dqE, dkg, dkd, dattn: 8,000 of the 12,600 MMAs at K = V = 128)
 // runs over 32 columns at a time, whose pieces of h_in, dh and v_new all warps cut and share.
-// B=8, S=4096, H=8, K=V=128: 1.02 ms (4.43 ms in float32 on the CUDA cores).
+// dqE, dkg and dkd are summed up by the tensor core: they leave in bf16, and dg, which takes their row sums, is no further from 64 bits
+// for it (2.3e-7 of its norm at 512 tokens, K = V = 128; 3.8e-7 in float32 on the CUDA cores; summed up with rounding 1.9e-7, and
+// this kernel 1.10 ms).  The [64, 64] sums, whose results are cut into pieces again, are rounded (gdn_mma.cuh).
+// B=8, S=4096, H=8, K=V=128: 1.03 ms (4.43 ms in float32 on the CUDA cores).
 template <int KB, int VB>
 __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs g) {
   extern __shared__ __align__(1024) uint8_t gdn_smem_raw[];
@@ -476,8 +464,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
     for (int ks = 0; ks < 4 * KB; ++ks) {
       const Frag4 bb = ld_b(tK, wc * 16, ks, L);
-      mma2(s2[0], s2[1], ld_a(tKb, wm * 16, ks, L).r, bb);
-      mma2(a2[0], a2[1], ld_a(tQ, wm * 16, ks, L).r, bb);
+      mma2_add(s2[0], s2[1], ld_a(tKb, wm * 16, ks, L).r, bb);
+      mma2_add(a2[0], a2[1], ld_a(tQ, wm * 16, ks, L).r, bb);
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -528,13 +516,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           if (ks < mrow[x]) continue;
-          Frag3x4 fa;
-#pragma unroll
-          for (int w3 = 0; w3 < 3; ++w3) {
-            const Frag4 f = ld_a_t(tA + w3 * kBox, ks * 16, mrow[x], L);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) fa.p[w3][e] = f.r[e];
-          }
+          const Frag3x4 fa = ld_a3_t(tA, kBox, ks * 16, mrow[x], L);
           mma_x6(acc[x][0], fa, b0);
           mma_x6(acc[x][1], fa, b1);
         }
@@ -614,16 +596,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
       for (int k2 = 0; k2 < 2; ++k2) {
         const int ks = vb * 2 + k2;
         const Frag4 fdo = ld_a(tDo, wm * 16, ks, L);
-        Frag3x4 fdvb, fvn;
-#pragma unroll
-        for (int w3 = 0; w3 < 3; ++w3) {
-          const Frag4 f = ld_a(tDvb + w3 * VB * kBox, wm * 16, ks, L), f2 = ld_a_t(base + M.svn + w3 * kHalfBox, k2 * 16, wm, L);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            fdvb.p[w3][e] = f.r[e];
-            fvn.p[w3][e] = f2.r[e];
-          }
-        }
+        const Frag3x4 fdvb = ld_a3(tDvb, VB * kBox, wm * 16, ks, L), fvn = ld_a3_t(base + M.svn, kHalfBox, k2 * 16, wm, L);
 #pragma unroll
         for (int cp = 0; cp < KB; ++cp) {
           const int np = wc * KB + cp;
@@ -631,18 +604,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
           for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(base + M.sh + w3 * KB * kHalfBox, k2 * 16, np, L, kHalfBox);
           mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[2]);
-          mma2_x6(dkb[2 * cp], dkb[2 * cp + 1], fdvb, hb[0], hb[1], hb[2]);
+          mma2_x6_acc(dkb[2 * cp], dkb[2 * cp + 1], fdvb, hb);
           mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[1]);
+          mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[0]);
 #pragma unroll
-          for (int w3 = 0; w3 < 3; ++w3) {
-            if (w3 == 0) mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[0]);
-            hb[w3] = ld_b_t(base + M.sdh + w3 * KB * kHalfBox, k2 * 16, np, L, kHalfBox);
-          }
-          mma2_x6(dk[2 * cp], dk[2 * cp + 1], fvn, hb[0], hb[1], hb[2]);
+          for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(base + M.sdh + w3 * KB * kHalfBox, k2 * 16, np, L, kHalfBox);
+          mma2_x6_acc(dk[2 * cp], dk[2 * cp + 1], fvn, hb);
         }
         if (active) {
-#pragma unroll
-          for (int w3 = 2; w3 >= 0; --w3) mma2(dat[0], dat[1], fdo.r, ld_b_t(base + M.svn + w3 * kHalfBox, k2 * 16, wc, L));
+          const Frag4 b[3] = {ld_b_t(base + M.svn, k2 * 16, wc, L), ld_b_t(base + M.svn + kHalfBox, k2 * 16, wc, L),
+                              ld_b_t(base + M.svn + 2 * kHalfBox, k2 * 16, wc, L)};
+          mma2_x3(dat[0], dat[1], fdo.r, b);
         }
       }
     }
@@ -685,14 +657,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   if (active) {
     for (int ks = 0; ks < 2 * nvb; ++ks) {
       const Frag4 bb = ld_b(tVb, wc * 16, ks, L);
-#pragma unroll
-      for (int w3 = 2; w3 >= 0; --w3) mma2(x1[0], x1[1], ld_a(tDvb + w3 * VB * kBox, wm * 16, ks, L).r, bb);
+      mma2_x3(x1[0], x1[1], ld_a3(tDvb, VB * kBox, wm * 16, ks, L), bb);
     }
 #pragma unroll
     for (int ks = 0; ks < 4 * KB; ++ks) {
       const Frag4 bb = ld_b(tKb, wc * 16, ks, L);
-#pragma unroll
-      for (int w3 = 2; w3 >= 0; --w3) mma2(x2[0], x2[1], ld_a(tStage + w3 * KB * kBox, wm * 16, ks, L).r, bb);
+      mma2_x3(x2[0], x2[1], ld_a3(tStage, KB * kBox, wm * 16, ks, L), bb);
     }
   }
   __syncthreads();   // dvb and dkg have been read: their places take T and X
@@ -720,14 +690,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       if (ks > wc) break;
-      Frag3x4 fx;
-#pragma unroll
-      for (int w3 = 0; w3 < 3; ++w3) {
-        const Frag4 f = ld_a(tStage + w3 * kBox, wm * 16, ks, L);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) fx.p[w3][e] = f.r[e];
-      }
-      mma2_x6(ds[0], ds[1], fx, ld_b(tA, wc * 16, ks, L), ld_b(tA + kBox, wc * 16, ks, L), ld_b(tA + 2 * kBox, wc * 16, ks, L));
+      const Frag4 b[3] = {ld_b(tA, wc * 16, ks, L), ld_b(tA + kBox, wc * 16, ks, L), ld_b(tA + 2 * kBox, wc * 16, ks, L)};
+      mma2_x6(ds[0], ds[1], ld_a3(tStage, kBox, wm * 16, ks, L), b);
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -755,7 +719,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
       if (lane < 4) colG[wm * C + wc * 16 + t * 8 + ec + e] = cs;
     }
 
-  // ---- dq += T k, dk += T^T q
+  // ---- dq += T k, dk += T^T q (rounded to bf16 next: accumulated by the tensor core, like dkb and dk below)
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll

@@ -39,12 +39,15 @@ __device__ __forceinline__ void f32_b(const float* m, int k0, int n0, int lane, 
   split3(p[8 * kSP], p[9 * kSP], b[0][1], b[1][1], b[2][1]);
 }
 __device__ __forceinline__ void mma_x6(float (&d)[4], const Frag3x4& a, const uint32_t (&b)[3][2]) {
-  mma(d, a.p[0], b[2][0], b[2][1]);
-  mma(d, a.p[2], b[0][0], b[0][1]);
-  mma(d, a.p[1], b[1][0], b[1][1]);
-  mma(d, a.p[0], b[1][0], b[1][1]);
-  mma(d, a.p[1], b[0][0], b[0][1]);
-  mma(d, a.p[0], b[0][0], b[0][1]);
+  float t[4];
+  zero4(t);
+  mma(t, a.p[0], b[2][0], b[2][1]);
+  mma(t, a.p[2], b[0][0], b[0][1]);
+  mma(t, a.p[1], b[1][0], b[1][1]);
+  mma(t, a.p[0], b[1][0], b[1][1]);
+  mma(t, a.p[1], b[0][0], b[0][1]);
+  mma(t, a.p[0], b[0][0], b[0][1]);
+  add4(d, t);
 }
 
 // A = (I + S)^-1 for the strictly lower S in sS; A (lower, exact zeros above the diagonal) goes to sA.  All threads, 256 or more.
@@ -138,16 +141,25 @@ __device__ __forceinline__ void unit_lower_inverse(const float* sS, float* sA, f
 }
 
 // Prefix sums of g and the decay factors of one chunk by warp 0: gates[0] = gcs, [1] = exp(gcs), [2] = exp(gcs_last - gcs).
+// The sum runs over the tokens in order, in every lane: the decay between two tokens is then off by the roundings between them
+// only.  (Prefixes by shuffles, each with roundings of its own, left the in-chunk attention 1.5 times as far from 64 bits.)
 __device__ __forceinline__ void chunk_gates(float* gates, float g0, float g1, int lane) {   // g of tokens 2*lane, 2*lane+1
-  float run = g0 + g1;
+  *reinterpret_cast<float2*>(gates + 2 * lane) = make_float2(g0, g1);
+  __syncwarp();
+  float last = 0.f, a = 0.f, b = 0.f;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float up = __shfl_up_sync(0xffffffffu, run, o);
-    if (lane >= o) run += up;
+  for (int i = 0; i < C / 4; ++i) {
+    const float4 x = *reinterpret_cast<const float4*>(gates + 4 * i);
+    last += x.x;
+    a = 2 * i == lane ? last : a;
+    last += x.y;
+    b = 2 * i == lane ? last : b;
+    last += x.z;
+    a = 2 * i + 1 == lane ? last : a;
+    last += x.w;
+    b = 2 * i + 1 == lane ? last : b;
   }
-  const float before = __shfl_up_sync(0xffffffffu, run, 1);
-  const float a = (lane > 0 ? before : 0.f) + g0, b = a + g1;
-  const float last = __shfl_sync(0xffffffffu, b, 31);
+  __syncwarp();
   gates[2 * lane] = a;
   gates[2 * lane + 1] = b;
   gates[C + 2 * lane] = __expf(a);
@@ -194,7 +206,7 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint4 v) {
 }
 
 // One CTA per chunk and head, two CTAs per SM.  About 1,300 MMAs per chunk (triangular blocks are skipped) and some 100 KB
-// in and out.  Latency-bound (ncu: 0.37 of the issue slots, no pipe above 0.4).  B=8, S=4096, H=8, K=V=128: 0.222 ms (0.79 ms
+// in and out.  Latency-bound (ncu: 0.37 of the issue slots, no pipe above 0.4).  B=8, S=4096, H=8, K=V=128: 0.225 ms (0.79 ms
 // with the products in float32 on the CUDA cores).
 template <int KB>
 __global__ void __launch_bounds__(kChunkThreads, 2)
@@ -292,7 +304,7 @@ fwd_chunk_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __res
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
         if (p > wm) break;
-        mma2(acc[2 * p], acc[2 * p + 1], a.r, ld_b(tK, p * 16, ks, L));
+        mma2_add(acc[2 * p], acc[2 * p + 1], a.r, ld_b(tK, p * 16, ks, L));
       }
     }
     uint32_t* at_out = reinterpret_cast<uint32_t*>(ws + W.attn) + chunk * 3 * C * C / 2;
@@ -355,6 +367,11 @@ fwd_chunk_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __res
     for (int ks = 0; ks < 4; ++ks) {
       // the 16-column load covers this warp's columns (KB = 2) or its and its neighbour's (KB = 1)
       const Frag4 bb = ld_b_t(tKb, ks * 16, KB == 2 ? warp : warp >> 1, L);
+      float t[4][KB][4];   // (products as Prod2 makes them; four chains side by side)
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int x = 0; x < KB; ++x) zero4(t[m][x]);
 #pragma unroll
       for (int w3 = 2; w3 >= 0; --w3)
 #pragma unroll
@@ -362,11 +379,15 @@ fwd_chunk_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __res
           if (m < ks) continue;
           const Frag4 a = ld_a(tPae + w3 * kBox, m * 16, ks, L);
           if constexpr (KB == 2) {
-            mma2(acc[m][0], acc[m][1], a.r, bb);
+            mma2(t[m][0], t[m][1], a.r, bb);
           } else {
-            mma(acc[m][0], a.r, (warp & 1) ? bb.r[2] : bb.r[0], (warp & 1) ? bb.r[3] : bb.r[1]);
+            mma(t[m][0], a.r, (warp & 1) ? bb.r[2] : bb.r[0], (warp & 1) ? bb.r[3] : bb.r[1]);
           }
         }
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int x = 0; x < KB; ++x) add4(acc[m][x], t[m][x]);
     }
 #pragma unroll
     for (int m = 0; m < 4; ++m)
@@ -395,13 +416,16 @@ fwd_chunk_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __res
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       const Frag4 a = ld_a_t(tV, ks * 16, warp, L);
+      Prod2 x[4];
 #pragma unroll
       for (int w3 = 2; w3 >= 0; --w3)
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           if (p < ks) continue;
-          mma2(acc[2 * p], acc[2 * p + 1], a.r, ld_b(tPa + w3 * kBox, p * 16, ks, L));
+          x[p].mul(a.r, ld_b(tPa + w3 * kBox, p * 16, ks, L));
         }
+#pragma unroll
+      for (int p = 0; p < 4; ++p) x[p].add_to(acc[2 * p], acc[2 * p + 1]);
     }
     uint4* out = reinterpret_cast<uint4*>(ws + W.ut) + ((chunk * W.v16 + blk) * 32 + lane) * 4;
 #pragma unroll
@@ -583,7 +607,7 @@ __device__ __forceinline__ void fwd_scan(const CUtensorMap& tm_w, const CUtensor
 #pragma unroll
       for (int t = 0; t < 2 * KT; ++t) dst[t * 32] = make_float4(hh[t][0], hh[t][1], hh[t][2], hh[t][3]);
     }
-    // h^T w^T with the old state
+    // h^T w^T with the old state (summed up by the tensor core, here and in rev_scan: with rounded sums the state is as far from 64 bits)
     float vn[8][4];
 #pragma unroll
     for (int t = 0; t < 8; ++t) zero4(vn[t]);
@@ -621,7 +645,7 @@ __device__ __forceinline__ void fwd_scan(const CUtensorMap& tm_w, const CUtensor
         for (int i = 0; i < 4; i += 2) {
           const Frag4 b0 = ld_b(st + St::q, pair_at(i) * 16, kq * KT + ks, L), b1 = ld_b(st + St::q, pair_at(i + 1) * 16, kq * KT + ks, L);
 #pragma unroll
-          for (int w3 = 2; w3 >= 0; --w3) {
+          for (int w3 = 2; w3 >= 0; --w3) {   // (o is rounded to bf16: accumulated by the tensor core)
             mma2(oo[2 * i], oo[2 * i + 1], hf[ks].p[w3], b0);
             mma2(oo[2 * i + 2], oo[2 * i + 3], hf[ks].p[w3], b1);
           }
@@ -668,11 +692,8 @@ __device__ __forceinline__ void fwd_scan(const CUtensorMap& tm_w, const CUtensor
         if (KS == 1 || t / OWN == kq) dst[t * 32] = make_float4(vn[t][0], vn[t][1], vn[t][2], vn[t][3]);
     }
     const float dec = gates[2 * C - 1];
-#pragma unroll
-    for (int t = 0; t < 2 * KT; ++t)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) hh[t][e] *= dec;
-    // attn v_new and h += (k exp(gcs_last - gcs))^T v_new, 16 tokens of v_new at a time
+    // attn v_new, 16 tokens of v_new at a time; the pieces of v_new exp(gcs_last - gcs)
+    Frag3x4 sf[4];
     float oa[OWN][4];
 #pragma unroll
     for (int t = 0; t < OWN; ++t) zero4(oa[t]);
@@ -684,27 +705,26 @@ __device__ __forceinline__ void fwd_scan(const CUtensorMap& tm_w, const CUtensor
       for (int i = 0; i < (STATES ? 0 : OP); ++i) {
         const int p = pair_at(i);
         if (p < ks) continue;   // attn is lower triangular: tokens 16*ks.. reach rows from 16*ks on
-        const Frag4 b0 = ld_b(st + St::at, p * 16, ks, L), b1 = ld_b(st + St::at + kBox, p * 16, ks, L),
-                    b2 = ld_b(st + St::at + 2 * kBox, p * 16, ks, L);
-        mma2_x6(oa[2 * i], oa[2 * i + 1], vf, b0, b1, b2);
+        const Frag4 b[3] = {ld_b(st + St::at, p * 16, ks, L), ld_b(st + St::at + kBox, p * 16, ks, L), ld_b(st + St::at + 2 * kBox, p * 16, ks, L)};
+        mma2_x6_acc(oa[2 * i], oa[2 * i + 1], vf, b);
       }
 #pragma unroll
       for (int t = 2 * ks; t < 2 * ks + 2; ++t) {
         const float2 e = *reinterpret_cast<const float2*>(gates + 2 * C + t * 8 + kc);
         vn[t][0] *= e.x; vn[t][1] *= e.y; vn[t][2] *= e.x; vn[t][3] *= e.y;
       }
-      split_acc(vn[2 * ks], vn[2 * ks + 1], vf);
-      constexpr int CW = KT >= 2 ? 2 : 1;   // column pairs side by side: independent accumulators between dependent MMAs
+      split_acc(vn[2 * ks], vn[2 * ks + 1], sf[ks]);
+    }
+    // h = h exp(gcs_last) + (k exp(gcs_last - gcs))^T v_new
+    constexpr int CW = KT >= 2 ? 2 : 1;   // column pairs side by side: independent accumulators between dependent MMAs
 #pragma unroll
-      for (int cp = 0; cp < KT; cp += CW) {
-        Frag4 kf[CW];
+    for (int cp = 0; cp < KT; cp += CW) {
+      float add[2 * CW][4];
+      chunk_sum<CW>(add, sf, [&](int ks, int x) { return ld_b_t(st + St::k, ks * 16, kq * KT + cp + x, L); });
 #pragma unroll
-        for (int x = 0; x < CW; ++x) kf[x] = ld_b_t(st + St::k, ks * 16, kq * KT + cp + x, L);
+      for (int t = 0; t < 2 * CW; ++t)
 #pragma unroll
-        for (int w3 = 2; w3 >= 0; --w3)
-#pragma unroll
-          for (int x = 0; x < CW; ++x) mma2(hh[2 * (cp + x)], hh[2 * (cp + x) + 1], vf.p[w3], kf[x]);
-      }
+        for (int e = 0; e < 4; ++e) hh[2 * cp + t][e] = fmaf(hh[2 * cp + t][e], dec, add[t][e]);
     }
     if constexpr (STATES) {   // (a quicker warp may not overwrite parts of v_new that a slower one still reads)
       __syncwarp();

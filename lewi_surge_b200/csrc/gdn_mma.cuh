@@ -9,7 +9,8 @@
 //
 // Float32 operands are cut into three bf16 pieces (8 + 8 + 8 mantissa bits, nothing of the 24 is lost), so a product of a
 // float32 and a bf16 operand is three MMAs and one of two float32 operands six (piece products below 2^-24 of the whole
-// are left out); all of them accumulate in float32.  Measured on a B200: one m16n8k16 per 8 cycles and scheduler.
+// are left out); all of them accumulate in float32, which the tensor core truncates (see Prod2).  Measured on a B200: one
+// m16n8k16 per 8 cycles and scheduler.
 #pragma once
 
 #include "common.cuh"
@@ -77,6 +78,29 @@ __device__ __forceinline__ Frag4 ld_a_t(uint32_t tile, int k0, int mp, LaneOff L
   return ldsm_t(tile + (mp >> 2) * stride + k0 * 128 + (L.n ^ ((mp & 3) << 5)));
 }
 
+// the three pieces of a float32 A operand, `stride` bytes apart
+__device__ __forceinline__ Frag3x4 ld_a3(uint32_t tile, int stride, int m0, int ks, LaneOff L) {
+  Frag3x4 f;
+#pragma unroll
+  for (int w3 = 0; w3 < 3; ++w3) {
+    const Frag4 x = ld_a(tile + w3 * stride, m0, ks, L);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f.p[w3][e] = x.r[e];
+  }
+  return f;
+}
+__device__ __forceinline__ Frag3x4 ld_a3_t(uint32_t tile, int stride, int k0, int mp, LaneOff L) {
+  Frag3x4 f;
+#pragma unroll
+  for (int w3 = 0; w3 < 3; ++w3) {
+    const Frag4 x = ld_a_t(tile + w3 * stride, k0, mp, L);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f.p[w3][e] = x.r[e];
+  }
+  return f;
+}
+
+__device__ __forceinline__ void zero4(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
 __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -88,21 +112,90 @@ __device__ __forceinline__ void mma2(float (&d0)[4], float (&d1)[4], const uint3
   mma(d0, a, b.r[0], b.r[1]);
   mma(d1, a, b.r[2], b.r[3]);
 }
+// A 16-deep product of both 8-column tiles that is to be added to float32 sums.  The tensor core truncates every sum that it makes
+// to float32 (a chain of n instructions comes out short by up to n * 2^-24 of itself, always towards zero), so a product starts
+// from zero, its pieces small to large, and is added with one rounding.  Error against 64 bits of the state, its gradient and that of
+// g, relative to their norm, where nothing is forgotten over 4096 tokens (K = V = 128): with the state as the accumulator 1.0e-5,
+// 9.6e-6, 1.0e-5; so 2.1e-7, 2.0e-7, 2.3e-7; in float32 on the CUDA cores 1.6e-6, 2.0e-7, 3.2e-7.
+__device__ __forceinline__ void add4(float (&d)[4], const float (&t)[4]) {   // two at a time, each rounded to nearest
+#pragma unroll
+  for (int e = 0; e < 4; e += 2)
+    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "+f"(d[e]), "+f"(d[e + 1]) : "f"(t[e]), "f"(t[e + 1]));
+}
+struct Prod2 {
+  float t0[4], t1[4];
+  __device__ __forceinline__ Prod2() {
+    zero4(t0);
+    zero4(t1);
+  }
+  __device__ __forceinline__ void mul(const uint32_t (&a)[4], const Frag4& b) { mma2(t0, t1, a, b); }
+  __device__ __forceinline__ void add_to(float (&d0)[4], float (&d1)[4]) const {
+    add4(d0, t0);
+    add4(d1, t1);
+  }
+};
+// bf16 A times bf16 B
+__device__ __forceinline__ void mma2_add(float (&d0)[4], float (&d1)[4], const uint32_t (&a)[4], const Frag4& b) {
+  Prod2 x;
+  x.mul(a, b);
+  x.add_to(d0, d1);
+}
 // float32 A (three pieces) times bf16 B
 __device__ __forceinline__ void mma2_x3(float (&d0)[4], float (&d1)[4], const Frag3x4& a, const Frag4& b) {
-  mma2(d0, d1, a.p[2], b);
-  mma2(d0, d1, a.p[1], b);
-  mma2(d0, d1, a.p[0], b);
+  Prod2 x;
+#pragma unroll
+  for (int w3 = 2; w3 >= 0; --w3) x.mul(a.p[w3], b);
+  x.add_to(d0, d1);
 }
-// float32 A times float32 B, three pieces each
-__device__ __forceinline__ void mma2_x6(float (&d0)[4], float (&d1)[4], const Frag3x4& a, const Frag4& b0, const Frag4& b1,
-                                        const Frag4& b2) {
-  mma2(d0, d1, a.p[0], b2);
-  mma2(d0, d1, a.p[2], b0);
-  mma2(d0, d1, a.p[1], b1);
-  mma2(d0, d1, a.p[0], b1);
-  mma2(d0, d1, a.p[1], b0);
-  mma2(d0, d1, a.p[0], b0);
+// s = the sum over the four 16-deep steps of a chunk of float32 A (steps `a`) times bf16 B (`b(step, x)`: column pair x).  What a
+// chunk adds to the state is summed up by itself and then added with one rounding, however many steps it has.
+template <int CW, class B>
+__device__ __forceinline__ void chunk_sum(float (&s)[2 * CW][4], const Frag3x4 (&a)[4], B b) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    Frag4 bf[CW];
+    Prod2 y[CW];
+#pragma unroll
+    for (int x = 0; x < CW; ++x) bf[x] = b(i, x);
+#pragma unroll
+    for (int w3 = 2; w3 >= 0; --w3)
+#pragma unroll
+      for (int x = 0; x < CW; ++x) y[x].mul(a[i].p[w3], bf[x]);
+#pragma unroll
+    for (int x = 0; x < CW; ++x) {
+      if (i == 0) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[2 * x][e] = y[x].t0[e];
+          s[2 * x + 1][e] = y[x].t1[e];
+        }
+      } else {
+        y[x].add_to(s[2 * x], s[2 * x + 1]);
+      }
+    }
+  }
+}
+// bf16 A times float32 B
+__device__ __forceinline__ void mma2_x3(float (&d0)[4], float (&d1)[4], const uint32_t (&a)[4], const Frag4 (&b)[3]) {
+  Prod2 x;
+#pragma unroll
+  for (int w3 = 2; w3 >= 0; --w3) x.mul(a, b[w3]);
+  x.add_to(d0, d1);
+}
+// float32 A times float32 B; `_acc`: accumulated by the tensor core, for what is rounded to bf16 next
+__device__ __forceinline__ void mma2_x6_acc(float (&d0)[4], float (&d1)[4], const Frag3x4& a, const Frag4 (&b)[3]) {
+  mma2(d0, d1, a.p[0], b[2]);
+  mma2(d0, d1, a.p[2], b[0]);
+  mma2(d0, d1, a.p[1], b[1]);
+  mma2(d0, d1, a.p[0], b[1]);
+  mma2(d0, d1, a.p[1], b[0]);
+  mma2(d0, d1, a.p[0], b[0]);
+}
+__device__ __forceinline__ void mma2_x6(float (&d0)[4], float (&d1)[4], const Frag3x4& a, const Frag4 (&b)[3]) {
+  Prod2 x;
+  mma2_x6_acc(x.t0, x.t1, a, b);
+  x.add_to(d0, d1);
 }
 
 // two floats -> three packed bf16 pairs, x = p0 + p1 + p2 exactly (up to float32 subnormals)
@@ -121,7 +214,6 @@ __device__ __forceinline__ void split_acc(const float (&t0)[4], const float (&t1
   split3(t1[2], t1[3], f.p[0][3], f.p[1][3], f.p[2][3]);
 }
 
-__device__ __forceinline__ void zero4(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 struct Dims {

@@ -303,3 +303,36 @@ def test_gdn_backward_takes_an_upstream_gradient_at_any_address(cuda):
   o, _ = seqmix.chunk_gated_delta_rule(*t)
   for a, w in zip(torch.autograd.grad(o, t, shifted, retain_graph=True), torch.autograd.grad(o, t, do)):
     assert torch.equal(a, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,h,kd", [(1, 2, 64), (2, 4, 128), (8, 8, 128), (13, 8, 128)])   # one, one, four and eight column groups per CTA
+def test_gdn_float32_results_come_from_rounded_sums(cuda, b, h, kd):
+  """Inputs whose values before every rounding to bf16 are exact (orthogonal rows of k with a few repeated, beta a power of two, no
+  decay, small whole q), so that the float32 results differ from 64 bits by float32 arithmetic alone.  Nothing is forgotten over
+  the 8 chunks: each adds to the state once, rounded by at most 2^-24.  (Sums truncated by the tensor core: 1.1e-6 to 1.7e-6.)"""
+  from lewi_surge_b200 import seqmix, _lib
+  from lewi_surge_b200._lib import ptr, stream
+  n, s = 8, 512
+  rng = np.random.default_rng(kd + b)
+  had = np.ones((1, 1))
+  while len(had) < kd:
+    had = np.block([[had, had], [had, -had]])
+  rows = np.stack([rng.permutation(kd)[:64] for _ in range(b * n * h)])
+  rows[:, 40:56] = rows[:, :16]
+  k = (had[rows] / (8 if kd == 64 else 16)).reshape(b, n, h, 64, kd).transpose(0, 1, 3, 2, 4).reshape(b, s, h, kd)
+  f = lambda *shape: rng.standard_normal(shape).astype(np.float32)
+  i = dict(q=rng.integers(-2, 3, (b, s, h, kd)), k=k, v=O.bf16_round(f(b, s, h, kd)), g=np.zeros((b, s, h)), beta=np.full((b, s, h), 2.0 ** -5),
+           h0=f(b, h, kd, kd), do=O.bf16_round(f(b, s, h, kd)), dhf=O.bf16_round(f(b, h, kd, kd)))
+  names = ("q", "k", "v", "g", "beta", "h0")
+  t = [to_dev(np.asarray(i[x], np.float32), torch.float32 if x in ("g", "h0") else torch.bfloat16, cuda).requires_grad_(True) for x in names]
+  o, hf = seqmix.chunk_gated_delta_rule(*t[:5], initial_state=t[5])
+  got = torch.autograd.grad((o, hf), t, (to_dev(i["do"], torch.bfloat16, cuda), to_dev(i["dhf"], torch.bfloat16, cuda)))
+  want = O.chunk_gated_delta_rule_bwd(*(i[x] for x in names[:5]), i["do"], i["dhf"], i["h0"])
+  norm_err = lambda a, w: float(np.linalg.norm(a.double().cpu().numpy() - w) / np.linalg.norm(w))
+  assert norm_err(got[3], want[3]) <= n * 2.0 ** -24 and norm_err(got[5], want[5]) <= n * 2.0 ** -24
+  _, want_h = _torch_chunked_delta_rule(*(torch.tensor(i[x], dtype=torch.float64) for x in names))
+  lib, out, state = _lib.load(), torch.empty_like(t[2]), torch.empty_like(t[5])   # (the state as the library has it: float32)
+  ws = torch.empty(int(lib.lewi_gdn_chunk_workspace_bytes(b, s, h, kd, kd)), dtype=torch.uint8, device=cuda)
+  _lib.check(lib.lewi_gdn_chunk_fwd(stream(), *(ptr(x.detach()) for x in t), ptr(out), ptr(state), ptr(ws), ws.numel(), b, s, h, kd, kd), "fwd")
+  assert norm_err(state, want_h.numpy()) <= n * 2.0 ** -24
