@@ -714,9 +714,10 @@ inline int route_chunk_slots(long long M, int k, bool tokens) {
   return (int)(t * k);
 }
 
+// Raises the kernel's limit on dynamic shared memory, once per device and whatever the first size is: the 48 KB that need no such
+// call are for dynamic and static memory together, and these kernels have 8 to 10 KB of the latter.
 template <class Kern>
 inline bool route_smem_ok(Kern kern, size_t smem, bool (&done)[64]) {
-  if (smem <= 48 * 1024) return true;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   if (done[dev]) return smem <= 200 * 1024;

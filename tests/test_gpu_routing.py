@@ -1,4 +1,8 @@
 """Router / sort kernels against the oracle: every integer output bit-exact."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -193,3 +197,26 @@ def test_router_keeps_a_nan_with_every_bit_set(cuda, t):
   assert np.array_equal(idx[0], np.arange(8)) and idx[1, 7] == 2 and np.array_equal(np.sort(idx[1]), np.arange(8))
   assert np.isnan(w[:2]).all() and np.isfinite(w[2:]).all()
   assert np.array_equal(to_np(tb.counts), np.full(8, t))
+
+
+def route_once(t, e, k):
+  """One routing call, a sort of t expert ids where k is 0, checked."""
+  from lewi_surge_b200 import layer, ops
+  cuda, rng = torch.device("cuda:0"), np.random.default_rng(t + e + k)
+  if k:
+    logits = rng.standard_normal((t, e)).astype(np.float32)
+    check_tables(layer.router_topk(to_dev(logits, torch.float32, cuda), k), logits, k, e)
+    return
+  idx = rng.integers(0, e, t).astype(np.int32)
+  order, _ = ops.sort_indices(to_dev(idx, torch.int32, cuda), e)
+  assert np.array_equal(to_np(order), np.argsort(idx, kind="stable"))
+
+
+@pytest.mark.parametrize("t,e,k", [(32768, 512, 8), (128, 512, 24), (64, 512, 32), (300_000, 512, 0)])
+def test_first_call_of_a_process_with_nearly_48_kb_of_shared_memory(cuda, t, e, k):
+  """Between 38 and 48 KB of dynamic shared memory the launch needs the raised limit for the sake of the kernels' static arrays; a larger
+  call before would have raised it, so each size gets a process of its own."""
+  here = os.path.dirname(os.path.abspath(__file__))
+  code = f"import sys; sys.path[:0] = [{os.path.dirname(here)!r}, {here!r}]; import test_gpu_routing as r; r.route_once({t}, {e}, {k})"
+  res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+  assert res.returncode == 0, res.stderr[-2000:]
