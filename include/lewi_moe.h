@@ -300,7 +300,9 @@ int lewi_causal_conv1d_bwd(void* stream, const void* x, const void* w, const voi
  * q, k bf16 [B,S,H,K]; v, o bf16 [B,S,H,V]; g f32 [B,S,H] (log decay, <= 0); beta bf16 [B,S,H];
  * h0 f32 [B,H,K,V] or null (zero state); h_final f32 [B,H,K,V] or null.  K <= 128 and a multiple of 8, V a
  * multiple of 8.  S need not be a multiple of 64 (the tail is padded with empty tokens, as the reference pads).
- * workspace: lewi_gdn_chunk_workspace_bytes(...) bytes (per-chunk u, w, in-chunk attention and cumulative decay).
+ * q, k, v and workspace are 16-byte aligned (LEWI_ERR_SHAPE otherwise); o may lie at any address of its type.
+ * workspace: lewi_gdn_chunk_workspace_bytes(...) bytes (per chunk of 64 tokens and head: q scaled, u, w, the in-chunk attention
+ * in three bf16 pieces, cumulative decay; 75 KB at K = V = 128).
  * The reference differentiates this function through JAX autodiff; lewi_gdn_chunk_bwd below is its gradient here. */
 int64_t lewi_gdn_chunk_workspace_bytes(int B, int S, int H, int K, int V);
 int lewi_gdn_chunk_fwd(void* stream, const void* q, const void* k, const void* v, const float* g, const void* beta,
@@ -310,9 +312,9 @@ int lewi_gdn_chunk_fwd(void* stream, const void* q, const void* k, const void* v
 /* Backward of lewi_gdn_chunk_fwd: gradients of q, k, v, beta (bf16, shapes of the inputs), g (f32 [B,S,H]) and,
  * optionally, of the initial state (dh0 f32 [B,H,K,V], may be null) from d_o (bf16 [B,S,H,V]) and, optionally, the
  * gradient of the final state (dh_final f32 [B,H,K,V], may be null).  fwd_workspace is the workspace lewi_gdn_chunk_fwd
- * filled for the same inputs (it holds u, w, the in-chunk attention and the cumulative decay of every chunk); workspace
- * is scratch of lewi_gdn_chunk_bwd_workspace_bytes (the state at the start of every chunk, which the first kernel
- * recomputes, and per-column-block partial sums that are added in a fixed order: no atomics, reproducible).  The
+ * filled for the same inputs; workspace is scratch of lewi_gdn_chunk_bwd_workspace_bytes (the state at the start and its
+ * gradient at the end of every chunk, v_new and its gradient, room for a copy of d_o; no atomics, reproducible).  q, k, v
+ * and both workspaces are 16-byte aligned; d_o, dq, dk and dv may lie at any address of their type.  The
  * forward pass's roundings to bf16 are kept in the values and differentiated as the identity, which is what automatic
  * differentiation of the reference's forward (modal/gdn_fast.py:37-113) does with its casts; the reference has no
  * backward of its own to compare with.  K, V <= 128, multiples of 8. */

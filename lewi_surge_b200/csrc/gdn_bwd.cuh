@@ -30,8 +30,9 @@ constexpr int kMaxVBwd = 128;
 // Backward workspace: accumulator tiles (32 lanes x 4 floats) of the transposed matrices, as the scans hold them:
 //   hs, dh [chunks][v16][8*kboxes][32] tiles of h_in^T and of dh^T (16 columns of V by 8 rows of the state each)
 //   vn, dv [chunks][v16][8][32]        tiles of v_new^T and dv_new^T (16 columns of V by 8 tokens)
+// and room for a copy of do, which the reverse scan fetches by TMA: made where do does not lie on a 16-byte boundary.
 struct BwdWs {
-  long long hs, dh, vn, dv, total;
+  long long hs, dh, vn, dv, d_o, total;
   int v16, kboxes;
 };
 __host__ __device__ inline BwdWs bwd_ws(const Dims& D) {
@@ -44,7 +45,8 @@ __host__ __device__ inline BwdWs bwd_ws(const Dims& D) {
   o.dh = state;
   o.vn = 2 * state;
   o.dv = 2 * state + rows;
-  o.total = 2 * (state + rows);
+  o.d_o = 2 * (state + rows);
+  o.total = o.d_o + ((long long)D.B * D.S * D.H * D.V * 2 + 255) / 256 * 256;
   return o;
 }
 
@@ -361,6 +363,16 @@ __device__ __forceinline__ uint32_t ld_shared32(uint32_t at) {
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
   return v;
 }
+// ANY: at any address of the element type (an instance of its own: the choice inside the kernel took 2 % of its time)
+template <bool ANY>
+__device__ __forceinline__ void st_pair(__nv_bfloat16* p, uint32_t v) {
+  if constexpr (ANY) {
+    reinterpret_cast<uint16_t*>(p)[0] = (uint16_t)v;
+    reinterpret_cast<uint16_t*>(p)[1] = (uint16_t)(v >> 16);
+  } else {
+    *reinterpret_cast<uint32_t*>(p) = v;
+  }
+}
 __device__ __forceinline__ float quad_sum(float v) {
   v += __shfl_xor_sync(0xffffffffu, v, 1);
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
@@ -373,7 +385,7 @@ __device__ __forceinline__ float quad_sum(float v) {
 // for it (2.3e-7 of its norm at 512 tokens, K = V = 128; 3.8e-7 in float32 on the CUDA cores; summed up with rounding 1.9e-7, and
 // this kernel 1.10 ms).  The [64, 64] sums, whose results are cut into pieces again, are rounded (gdn_mma.cuh).
 // B=8, S=4096, H=8, K=V=128: 1.03 ms (4.43 ms in float32 on the CUDA cores).
-template <int KB, int VB>
+template <int KB, int VB, bool ANY>
 __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs g) {
   extern __shared__ __align__(1024) uint8_t gdn_smem_raw[];
   constexpr BwdSmem M = bwd_smem(KB, VB);
@@ -537,7 +549,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
               const uint32_t vv = *reinterpret_cast<const uint32_t*>(g.v + row_off(r) * V + c);
               rb = fmaf(d0, bf16_lo(vv), rb);
               rb = fmaf(d1, bf16_hi(vv), rb);
-              *reinterpret_cast<uint32_t*>(g.dv + row_off(r) * V + c) = pack_bf16(d0 * be, d1 * be);
+              st_pair<ANY>(g.dv + row_off(r) * V + c, pack_bf16(d0 * be, d1 * be));
             }
           }
           rb = quad_sum(rb);
@@ -742,7 +754,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int r = wm * 16 + er + 8 * e, c = wc * 16 * KB + t * 8 + ec;
-      if (in_seq(r) && c < K) *reinterpret_cast<uint32_t*>(g.dq + row_off(r) * K + c) = pack_bf16(dq[t][2 * e] * scale, dq[t][2 * e + 1] * scale);
+      if (in_seq(r) && c < K) st_pair<ANY>(g.dq + row_off(r) * K + c, pack_bf16(dq[t][2 * e] * scale, dq[t][2 * e + 1] * scale));
     }
   __syncthreads();
 
@@ -776,8 +788,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
       rb = fmaf(dkb[t][2 * e], bf16_lo(kk), rb);
       rb = fmaf(dkb[t][2 * e + 1], bf16_hi(kk), rb);
       if (in_seq(r) && c < K)
-        *reinterpret_cast<uint32_t*>(g.dk + row_off(r) * K + c) =
-            pack_bf16(fmaf(dkb[t][2 * e], be, dk[t][2 * e]), fmaf(dkb[t][2 * e + 1], be, dk[t][2 * e + 1]));
+        st_pair<ANY>(g.dk + row_off(r) * K + c, pack_bf16(fmaf(dkb[t][2 * e], be, dk[t][2 * e]), fmaf(dkb[t][2 * e + 1], be, dk[t][2 * e + 1])));
     }
     rb = quad_sum(rb);
     if ((lane & 3) == 0) dbK[wc * C + r] = rb;
@@ -843,13 +854,13 @@ inline int launch_scans(cudaStream_t st, const RevMaps& m, const ScanArgs& fwd, 
   return launch_scans_side<KB, NG, KS, 2>(st, m, fwd, rev);
 }
 
-template <int KB, int VB>
+template <int KB, int VB, bool ANY>
 inline int launch_bwd_chunk(cudaStream_t st, const BwdArgs& a) {
   static bool done[64] = {false};
   constexpr int smem = bwd_smem(KB, VB).total;
   static_assert(smem <= 227 * 1024, "shared memory of the chunk kernel");
-  if (!allow_smem(bwd_chunk_kernel<KB, VB>, smem, done)) return LEWI_ERR_CUDA;
-  bwd_chunk_kernel<KB, VB><<<dim3((unsigned)a.D.N, (unsigned)a.D.H, (unsigned)a.D.B), kBwdThreads, smem, st>>>(a);
+  if (!allow_smem(bwd_chunk_kernel<KB, VB, ANY>, smem, done)) return LEWI_ERR_CUDA;
+  bwd_chunk_kernel<KB, VB, ANY><<<dim3((unsigned)a.D.N, (unsigned)a.D.H, (unsigned)a.D.B), kBwdThreads, smem, st>>>(a);
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }
@@ -860,6 +871,13 @@ inline int backward(cudaStream_t st, const void* k, const void* v, const void* b
                     float* dh0, const Dims& D) {
   const FwdWs FW = fwd_ws(D);
   const BwdWs BW = bwd_ws(D);
+  if ((reinterpret_cast<uintptr_t>(d_o) & 15u) != 0) {
+    if (cudaMemcpyAsync(bws + BW.d_o, d_o, (size_t)D.B * D.S * D.H * D.V * 2, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return LEWI_ERR_CUDA;
+    }
+    d_o = bws + BW.d_o;
+  }
   const float* gates = reinterpret_cast<const float*>(fws + FW.gates);
   const ScanArgs sa{reinterpret_cast<const uint32_t*>(fws + FW.ut), gates, h0, nullptr, nullptr, reinterpret_cast<float4*>(bws + BW.hs),
                     reinterpret_cast<float4*>(bws + BW.vn), FW.v16, D};
@@ -887,7 +905,9 @@ inline int backward(cudaStream_t st, const void* k, const void* v, const void* b
   using bf = __nv_bfloat16;
   const BwdArgs ba{reinterpret_cast<const bf*>(k), reinterpret_cast<const bf*>(v), reinterpret_cast<const bf*>(beta), reinterpret_cast<const bf*>(d_o),
                    fws, bws, reinterpret_cast<bf*>(dq), reinterpret_cast<bf*>(dk), reinterpret_cast<bf*>(dv), reinterpret_cast<bf*>(dbeta), dg, D};
-  return D.V <= 64 ? launch_bwd_chunk<KB, 1>(st, ba) : launch_bwd_chunk<KB, 2>(st, ba);
+  const bool any = ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 3u) != 0;
+  if (D.V <= 64) return any ? launch_bwd_chunk<KB, 1, true>(st, ba) : launch_bwd_chunk<KB, 1, false>(st, ba);
+  return any ? launch_bwd_chunk<KB, 2, true>(st, ba) : launch_bwd_chunk<KB, 2, false>(st, ba);
 }
 
 }  // namespace gdn

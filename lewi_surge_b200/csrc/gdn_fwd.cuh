@@ -768,7 +768,7 @@ __device__ __forceinline__ void fwd_scan(const CUtensorMap& tm_w, const CUtensor
     for (int i = 0; i < OP; ++i) {
       const long long t = (long long)n * C + pair_at(i) * 16 + (lane >> 1);
       const uint4 val = *reinterpret_cast<const uint4*>(my_out + (i * 16 + (lane >> 1)) * kOutPitch + (lane & 1) * 16);
-      if (t < D.S && vcol < D.V) st_v4(a.o + (((long long)b * D.S + t) * D.H + h) * D.V + vcol, val);
+      if (t < D.S && vcol < D.V) st_out8(a.o + (((long long)b * D.S + t) * D.H + h) * D.V + vcol, val, a.o);
     }
     __syncwarp();
   }

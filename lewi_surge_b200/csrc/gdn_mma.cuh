@@ -214,6 +214,16 @@ __device__ __forceinline__ void split_acc(const float (&t0)[4], const float (&t1
   split3(t1[2], t1[3], f.p[0][3], f.p[1][3], f.p[2][3]);
 }
 
+// An output may lie at any address of its element type (2 bytes): whole pieces where its base allows it.
+__device__ __forceinline__ void st_out8(__nv_bfloat16* p, uint4 v, const __nv_bfloat16* base) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) == 0) {
+    st_v4(p, v);
+    return;
+  }
+  const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) reinterpret_cast<uint16_t*>(p)[i] = (uint16_t)(x[i >> 1] >> ((i & 1) * 16));
+}
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 struct Dims {

@@ -1206,7 +1206,7 @@ int lewi_gdn_chunk_fwd(void* stream, const void* q, const void* k, const void* v
   if (!q || !k || !v || !g || !beta || !o || !workspace || B <= 0 || S <= 0 || H <= 0 || K <= 0 || V <= 0) return LEWI_ERR_ARG;
   if (K > gdn::kMaxK || V > gdn::kMaxV) return LEWI_ERR_LIMIT;
   if (K % 8 != 0 || V % 8 != 0) return LEWI_ERR_SHAPE;
-  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(workspace)) return LEWI_ERR_SHAPE;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(workspace)) return LEWI_ERR_SHAPE;
   if (workspace_bytes < lewi_gdn_chunk_workspace_bytes(B, S, H, K, V)) return LEWI_ERR_WORKSPACE;
   const gdn::Dims D{B, S, H, K, V, (S + gdn::C - 1) / gdn::C};
   if ((long long)B * D.N * H > gdn::kMaxChunks || H > 65535 || B > 65535) return LEWI_ERR_LIMIT;
@@ -1230,9 +1230,7 @@ int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v
   if (B <= 0 || S <= 0 || H <= 0 || K <= 0 || V <= 0) return LEWI_ERR_ARG;
   if (K > gdn::kMaxK || V > gdn::kMaxVBwd) return LEWI_ERR_LIMIT;
   if (K % 8 != 0 || V % 8 != 0) return LEWI_ERR_SHAPE;
-  if (!aligned16(k) || !aligned16(v) || !aligned16(d_o) || !aligned16(fwd_workspace) || !aligned16(workspace) || !aligned16(dq) ||
-      !aligned16(dk) || !aligned16(dv))
-    return LEWI_ERR_SHAPE;
+  if (!aligned16(k) || !aligned16(v) || !aligned16(fwd_workspace) || !aligned16(workspace)) return LEWI_ERR_SHAPE;
   if (fwd_workspace_bytes < lewi_gdn_chunk_workspace_bytes(B, S, H, K, V)) return LEWI_ERR_WORKSPACE;
   if (workspace_bytes < lewi_gdn_chunk_bwd_workspace_bytes(B, S, H, K, V)) return LEWI_ERR_WORKSPACE;
   const gdn::Dims D{B, S, H, K, V, (S + gdn::C - 1) / gdn::C};

@@ -84,8 +84,6 @@ class _ChunkGatedDeltaRule(torch.autograd.Function):
     b, s, h, kd = k.shape
     vd = v.shape[-1]
     d_o = d_o.to(torch.bfloat16).contiguous() if d_o is not None else torch.zeros_like(v)
-    if d_o.data_ptr() % 16:   # a view into another tensor: the kernels read whole 16-byte pieces
-      d_o = d_o.clone()
     d_hf = d_hf.to(torch.float32).contiguous() if d_hf is not None else None
     bws_bytes = int(lib.lewi_gdn_chunk_bwd_workspace_bytes(b, s, h, kd, vd))
     if bws_bytes < 0:

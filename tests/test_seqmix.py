@@ -336,3 +336,36 @@ def test_gdn_float32_results_come_from_rounded_sums(cuda, b, h, kd):
   ws = torch.empty(int(lib.lewi_gdn_chunk_workspace_bytes(b, s, h, kd, kd)), dtype=torch.uint8, device=cuda)
   _lib.check(lib.lewi_gdn_chunk_fwd(stream(), *(ptr(x.detach()) for x in t), ptr(out), ptr(state), ptr(ws), ws.numel(), b, s, h, kd, kd), "fwd")
   assert norm_err(state, want_h.numpy()) <= n * 2.0 ** -24
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,s,h,kd,vd", [(1, 70, 2, 32, 24), (2, 65, 8, 128, 128)])
+def test_gdn_takes_outputs_and_upstream_gradients_at_any_address(cuda, b, s, h, kd, vd):
+  """o, d_o, dq, dk and dv one element past a 16-byte boundary, through the C entries: the same bits, and nothing beside them."""
+  from lewi_surge_b200 import _lib
+  from lewi_surge_b200._lib import ptr, stream
+  lib, bf = _lib.load(), torch.bfloat16
+  i = _gdn_inputs(b, s, h, kd, vd, seed=9)
+  q, k, v, g, beta, h0, do, dhf = (to_dev(i[n], torch.float32 if n in ("g", "h0", "dhf") else bf, cuda)
+                                   for n in ("q", "k", "v", "g", "beta", "h0", "do", "dhf"))
+
+  def run(shift):
+    place = lambda like: torch.full((like.numel() + 16,), 7.0, dtype=bf, device=cuda)
+    bufs = dict(o=place(do), dq=place(q), dk=place(k), dv=place(v), do=place(do))
+    at = lambda n: bufs[n][shift:]
+    bufs["do"][shift:shift + do.numel()] = do.reshape(-1)
+    ws = torch.empty(int(lib.lewi_gdn_chunk_workspace_bytes(b, s, h, kd, vd)), dtype=torch.uint8, device=cuda)
+    bws = torch.empty(int(lib.lewi_gdn_chunk_bwd_workspace_bytes(b, s, h, kd, vd)), dtype=torch.uint8, device=cuda)
+    hf, dg, db, dh0 = (torch.empty_like(t) for t in (h0, g, beta, h0))
+    _lib.check(lib.lewi_gdn_chunk_fwd(stream(), ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(h0), ptr(at("o")), ptr(hf), ptr(ws), ws.numel(),
+                                      b, s, h, kd, vd), "fwd")
+    _lib.check(lib.lewi_gdn_chunk_bwd(stream(), ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(h0), ptr(at("do")), ptr(dhf), ptr(ws), ws.numel(),
+                                      ptr(bws), bws.numel(), ptr(at("dq")), ptr(at("dk")), ptr(at("dv")), ptr(dg), ptr(db), ptr(dh0), b, s, h,
+                                      kd, vd), "bwd")
+    for n, t in bufs.items():
+      end = shift + t.numel() - 16
+      assert torch.all(t[:shift] == 7) and torch.all(t[end:] == 7), n
+    return [bufs[n][shift:shift + bufs[n].numel() - 16] for n in ("o", "dq", "dk", "dv")] + [hf, dg, db, dh0]
+
+  for shift in (1, 2):
+    assert all(torch.equal(x, y) for x, y in zip(run(0), run(shift)))
