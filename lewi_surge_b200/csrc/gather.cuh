@@ -220,7 +220,11 @@ __global__ void __launch_bounds__(kGatherThreads) gather_reduce_kernel(
 // The same for few rows, same bits: a warp takes 32 vectors of one row of `out` and has eight rows of y in flight.  The kernel
 // above walks the k rows of a token one trip to memory after the other, which is what a small call takes
 // (8 tokens, k = 6, d = 1024: 10.2 us, here 4.1; 64 tokens, k = 8, d = 2048: 23 and 5.1 us; 1000 tokens, k = 6: 10.7 and 6.1).
-// Taken while all its warps are resident at once; from there on the row kernel has enough in flight and reads positions once.
+// It reads positions and weights once per 32 vectors, so where the trips are few (small k) or short rows give the row kernel warps
+// enough, that one is quicker from some size on.  Measured line between them (k 1 to 12, d 128 to 4096, bf16 and float32, 300 to
+// 9500 warps, sources in L2): gather_reduce_few() picks the quicker one within 1 % on average and never one more than 5 % slower.
+// Either side of it, in us, this kernel first: bf16 d = 1024, k = 1: 592 rows 2.4 and 2.3, 2368 rows 5.2 and 2.7; k = 6: 1184 rows
+// 4.0 and 4.6, 2368 rows 6.5 and 5.2; d = 2048, k = 8: 1184 rows 7.0 and 8.6.
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(kGatherThreads) gather_reduce_few_kernel(
     const TI* __restrict__ y, const int32_t* __restrict__ pos, const float* __restrict__ w,
@@ -286,6 +290,13 @@ __global__ void __launch_bounds__(kGatherThreads) gather_reduce_few_kernel(
   } else {
     *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]));
   }
+}
+
+// Whether a call of `warps` warps goes to the kernel above (see there): more trips (k) and longer rows (d) move the line up.
+inline bool gather_reduce_few(long long warps, int k, int d) {
+  const int ke = k < 7 ? k : 7;   // (from eight source rows on, in flight at once, more of them do not help)
+  const long long line = 4ll * num_sms() * (ke - 1) + (long long)d * (ke + 1) / 2, most = 64ll * num_sms();
+  return warps <= (line < most ? line : most);
 }
 
 // out[t,j] = <g[t], y[pos[t,j]]>.

@@ -142,8 +142,8 @@ def test_dispatch_rows_equals_the_row_gather(cuda, t, e, k, d, skew):
                                        (torch.float32, torch.bfloat16)])
 @pytest.mark.parametrize("k", [1, 8, 9, 32])
 def test_gather_reduce_of_few_rows_gives_the_bits_of_many(cuda, dtype, out, k):
-  """A call of up to one resident wave of warps takes another kernel than a larger one: 1, 3 and 700 rows against the same rows
-  of a call of 10000, with weights, both addends, absent rows and a row length that fills no warp."""
+  """Few rows (how many depends on k and d: here up to 132 at k = 1 and 2300 at k >= 8) take another kernel than many: 1, 3 and 700
+  rows against the same rows of a call of 10000, with weights, both addends, absent rows and a row length that fills no warp."""
   from lewi_surge_b200 import ops
   d, n, m = 264, 10000, 500
   gen = torch.Generator(device=cuda).manual_seed(k)
