@@ -89,10 +89,12 @@ __global__ void __launch_bounds__(kGatherThreads) gather_rows_kernel(
 // (row_slot[r] < 0) become zero rows.  Every output row has exactly one writer, so this is the same function as
 // the row gather out[r] = x[row_slot[r] / k] -- but each source row is read once instead of k times at k distant
 // moments, which keeps the read side at T rows of DRAM traffic however large the source is against the L2.
-// A warp zeroes a few rows at a time: at decode sizes nearly all rows are such rows
-// (8 tokens over 128 experts: 6.1 MB of zeros; 13 us with 32 rows per warp, 7 us with 4).
+// A warp looks at ZR rows at a time for those to zero: 4 while no warp of the grid looks more than twice (kZeroRows), since at decode
+// sizes nearly all rows are such rows (8 tokens over 128 experts: 6.1 MB of zeros; 13 us with 32 rows per warp, 7 us with 4);
+// 32 beyond, where hardly any are (k = 6, d = 256: 16,384 tokens over 16 experts 9.3 us with 4 and 9.8 with 32, 49,152 34 and 32,
+// 65,536 over 128 48 and 45).
 constexpr int kZeroRows = 4;
-template <int VPL>
+template <int VPL, int ZR>
 __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
     const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
     __nv_bfloat16* __restrict__ out, long long n_tokens, int k, int d, long long out_rows,
@@ -126,9 +128,9 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
     }
   }
   // zero rows of the padded layout
-  for (long long r0 = warp0 * kZeroRows; r0 < rows; r0 += n_warps * kZeroRows) {
+  for (long long r0 = warp0 * ZR; r0 < rows; r0 += n_warps * ZR) {
     const long long r = r0 + lane;
-    const unsigned empty = __ballot_sync(0xffffffffu, lane < kZeroRows && r < rows && row_slot[r] < 0);
+    const unsigned empty = __ballot_sync(0xffffffffu, lane < ZR && r < rows && row_slot[r] < 0);
     for (unsigned m = empty; m != 0; m &= m - 1) {
       const long long rr = r0 + (__ffs(m) - 1);
       for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + rr * d) + vi, make_uint4(0, 0, 0, 0));

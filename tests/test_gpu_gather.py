@@ -117,7 +117,8 @@ def test_full_size_dispatch_combine_round_trip(cuda):
   assert torch.equal(back, x.float() * k)
 
 
-@pytest.mark.parametrize("t,e,k,d,skew", [(300, 8, 2, 128, False), (4096, 64, 6, 1024, False), (5000, 128, 6, 256, True)])
+@pytest.mark.parametrize("t,e,k,d,skew", [(300, 8, 2, 128, False), (4096, 64, 6, 1024, False), (5000, 128, 6, 256, True),
+                                          (30000, 16, 6, 136, False)])
 def test_dispatch_rows_equals_the_row_gather(cuda, t, e, k, d, skew):
   """The token-order dispatch writes exactly what the gather through row_slot writes, zero padding rows included."""
   from lewi_surge_b200 import layer, ops, _lib
