@@ -1160,7 +1160,11 @@ int lewi_causal_conv1d_fwd(void* stream, const void* x, const void* w, void* y, 
   const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(w);
   __nv_bfloat16* yb = reinterpret_cast<__nv_bfloat16*>(y);
   cudaStream_t st = as_stream(stream);
-  LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<KT><<<grid, kConvThreads, 0, st>>>(xb, wb, yb, B, T, C)));
+  if (T <= 2) {
+    LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<KT, 1><<<grid, kConvThreads, 0, st>>>(xb, wb, yb, B, T, C)));
+  } else {
+    LEWI_DISPATCH_TAPS(K, (causal_conv1d_kernel<KT, kConvBatch<KT>><<<grid, kConvThreads, 0, st>>>(xb, wb, yb, B, T, C)));
+  }
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }

@@ -47,12 +47,13 @@ __device__ __forceinline__ uint4 conv_fetch(const __nv_bfloat16* __restrict__ p,
   return t >= 0 && t < t_end ? ld_nc_v4(p + (long long)t * C) : make_uint4(0, 0, 0, 0);
 }
 
-// B=8, T=4096, C=4096, 4 taps (0.54 GB): 88 us, 6.1 TB/s (105 us with one vector requested at a time).
-template <int KT>
+// B=8, T=4096, C=4096, 4 taps (0.54 GB): 88 us, 6.1 TB/s (105 us with one vector requested at a time).  NB = kConvBatch<KT>, or 1 for
+// one or two steps, since the rest of a batch is worked through for nothing (1024 channels, 4 taps, a batch of 8 and of 1: one
+// step 2.0 and 1.7 us, two 2.1 and 1.8, four 2.2 and 2.1, seven 2.3 and 2.5; 8 taps, four 2.2 and 2.6).
+template <int KT, int NB>
 __global__ void __launch_bounds__(kConvThreads) causal_conv1d_kernel(const __nv_bfloat16* __restrict__ x,
                                                                      const __nv_bfloat16* __restrict__ w,
                                                                      __nv_bfloat16* __restrict__ y, int B, int T, int C) {
-  constexpr int NB = kConvBatch<KT>;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;      // channel vector
   if (v >= C / 8) return;
   const int c0 = v * 8, b = blockIdx.z, t0 = blockIdx.y * kConvRun, t_end = min(t0 + kConvRun, T);
