@@ -4,9 +4,11 @@
 //   up to kFusedTokens tokens   route_fused_kernel: one CTA does everything;
 //   otherwise                   route_chunk_kernel: one CTA per chunk of slots ((soft-max + top-k + renormalise when fed
 //                               logits) and a histogram of the chunk's expert ids), then route_rank_kernel: every CTA adds
-//                               up the histograms of all chunks (at most one chunk per SM, so that is a few loads per thread
-//                               out of L2 and spares a launch for a scan), derives the offsets and ranks its own slots ->
-//                               pos / order / padded row / slot-of-row.
+//                               up the histograms of all chunks (one chunk per SM up to 4.8 million slots, so that is a few loads
+//                               per thread out of L2 and spares a launch for a scan), derives the offsets and ranks its own
+//                               slots -> pos / order / padded row / slot-of-row.  A chunk holds at most 32,768 slots, so with
+//                               the slots the chunks become more and those loads grow with their square: beyond kScanChunks
+//                               of them route_scan_kernel comes in between and leaves every chunk's prefix and the totals.
 // The result equals sort_indices() of the reference (modal/moe_permute.py:240-264): a stable sort
 // of slots i = t*k + j by expert id, order[p] = slot at sorted position p, pos = inverse of order.
 #pragma once
@@ -20,6 +22,7 @@ constexpr int kRouteWarps = kRouteThreads / kWarp;
 constexpr int kFusedTokens = 128;       // one CTA routes up to this many tokens (two rounds of 16 warps x 4 tokens)
 constexpr int kMinChunkSlots = 128;     // lewi_route_workspace_bytes counts on it
 constexpr int kMaxChunkSlots = 32768;   // a chunk's expert ids and 17 rows of 512 counters fit in 200 KB of shared memory
+constexpr int kScanChunks = 512;        // see route_scan_kernel
 constexpr int kMaxExperts = 512;
 constexpr int kMaxTopK = 32;
 
@@ -379,12 +382,41 @@ __device__ __forceinline__ void rank_slots(const RouteTables& t, const int* s_e,
   }
 }
 
+// Histograms of all chunks -> what the earlier chunks hold, and the totals as row n_chunks: a CTA per 32 experts, whose warps take a run
+// of chunks each, add it up and walk it again.  Sorting over 512 / 128 / 16 experts, without and with it (chunks of 32,768): 306 chunks
+// 0.35 and 0.33 / 0.31 and 0.30 / 0.202 and 0.207 ms, 611 chunks 0.71 and 0.61 / 0.58 and 0.56 / 0.398 and 0.399, 300 million slots 35
+// and 9.2 / 12.9 and 8.7 / 5.3 and 4.7, 1.5 billion 1007 and 46 / 220 and 42.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads) route_scan_kernel(int32_t* chunk_hist, int n_chunks, int E) {
+  constexpr int NW = kScanThreads / kWarp;
+  __shared__ int s_sum[NW][kWarp];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * kWarp + lane;
+  const int per = (n_chunks + NW - 1) / NW, c0 = min(warp * per, n_chunks), c1 = min(c0 + per, n_chunks);
+  const bool live = e < E;
+  int32_t* col = chunk_hist + e;
+  int sum = 0;
+#pragma unroll 8
+  for (int c = c0; c < c1; ++c) sum += live ? col[(long long)c * E] : 0;
+  s_sum[warp][lane] = sum;
+  __syncthreads();
+  int run = 0;
+  for (int w = 0; w < warp; ++w) run += s_sum[w][lane];
+#pragma unroll 8
+  for (int c = c0; c < c1; ++c) {
+    const int h = live ? col[(long long)c * E] : 0;
+    if (live) col[(long long)c * E] = run;
+    run += h;
+  }
+  if (warp == NW - 1 && live) col[(long long)n_chunks * E] = run;
+}
+
 struct RouteRankArgs {
   RouteTables t;
   const int32_t* flat;        // [M] expert id per slot
-  const int32_t* chunk_hist;  // [n_chunks, E]
+  const int32_t* chunk_hist;  // [n_chunks, E], or scanned: [n_chunks + 1, E]
   const float* chunk_probs;   // [n_chunks, E] or null
   int n_chunks, chunk_slots;
+  bool scanned;
 };
 
 __global__ void __launch_bounds__(kRouteThreads) route_rank_kernel(RouteRankArgs a) {
@@ -407,7 +439,12 @@ __global__ void __launch_bounds__(kRouteThreads) route_rank_kernel(RouteRankArgs
   __syncthreads();
   // totals of all chunks and of the earlier ones: an expert's chunks are dealt over kRouteThreads / E threads
   const int parts = kRouteThreads / E, e = tid % E, part = tid / E;
-  if (part < parts) {
+  if (a.scanned) {
+    if (tid < E) {
+      s_base[tid] = a.chunk_hist[(long long)chunk * E + tid];
+      s_cnt[tid] = a.chunk_hist[(long long)a.n_chunks * E + tid];
+    }
+  } else if (part < parts) {
     int tot = 0, before = 0;
 #pragma unroll 8
     for (int c = part; c < a.n_chunks; c += parts) {
@@ -699,19 +736,19 @@ __global__ void __launch_bounds__(256) split3_bf16_kernel(const float* __restric
 
 // ------------------------------------------------------------------------------------------------ host
 
-// Slots per chunk: one chunk per SM (see route_rank_kernel) until a chunk no longer fits in shared memory, whole tokens when
-// fed logits (k slots each).
+// Slots per chunk: one chunk per SM (see route_rank_kernel), or as few per SM as fit in shared memory, the same number on each (five
+// million slots in chunks of 32,768 are one chunk per SM and five more: over 16 experts 127 us, so 70); whole tokens when fed logits
+// (k slots each).
 inline int route_chunk_slots(long long M, int k, bool tokens) {
-  const long long per = (M + num_sms() - 1) / num_sms();
-  if (!tokens) {
-    const long long s = (per + 255) / 256 * 256;
-    return (int)(s < 256 ? 256 : (s > kMaxChunkSlots ? kMaxChunkSlots : s));
-  }
-  long long t = (per + k - 1) / k;                           // tokens: whole rounds of the CTA's 16 warps
-  t = (t + kRouteWarps - 1) / kRouteWarps * kRouteWarps;
-  if (t * k < kMinChunkSlots) t = (kMinChunkSlots + k - 1) / k;
-  if (t * k > kMaxChunkSlots) t = kMaxChunkSlots / k / kRouteWarps * kRouteWarps;
-  return (int)(t * k);
+  const long long unit = tokens ? (long long)k * kRouteWarps : 256;   // tokens: whole rounds of the CTA's 16 warps
+  const long long most = kMaxChunkSlots / unit * unit;
+  const long long per_sm = (M + num_sms() - 1) / num_sms(), rounds = (per_sm + most - 1) / most;
+  const long long per = rounds > 1 ? (M + num_sms() * rounds - 1) / (num_sms() * rounds) : per_sm;
+  long long s = (per + unit - 1) / unit * unit;
+  if (s > most) s = most;
+  if (s < unit) s = unit;
+  if (tokens && s < kMinChunkSlots) s = (kMinChunkSlots + k - 1) / k * k;
+  return (int)s;
 }
 
 // Raises the kernel's limit on dynamic shared memory, once per device and whatever the first size is: the 48 KB that need no such
@@ -786,7 +823,8 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
   } while (0)
   const int chunk_slots = route_chunk_slots(M, k, logits != nullptr);
   const int n_chunks = (int)((M + chunk_slots - 1) / chunk_slots);
-  const long long need = (long long)n_chunks * E * 8;
+  const bool scanned = n_chunks > kScanChunks;
+  const long long hist_rows = n_chunks + (scanned ? 1 : 0), need = (hist_rows + n_chunks) * E * 4;
   if (ws == nullptr || ws_bytes < need) return LEWI_ERR_WORKSPACE;   // also where the one-CTA path would not touch it
   if (logits != nullptr && T > 0 && T <= kFusedTokens) {
     const RouteFusedArgs fa{t, logits, topk_idx, topk_w, mpad, k};
@@ -794,7 +832,7 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
     return LEWI_OK;
   }
   int32_t* chunk_hist = reinterpret_cast<int32_t*>(ws);
-  float* chunk_probs = reinterpret_cast<float*>(chunk_hist + (long long)n_chunks * E);
+  float* chunk_probs = reinterpret_cast<float*>(chunk_hist + hist_rows * E);
   RouteChunkArgs ca;
   ca.logits = logits;
   ca.flat_in = flat_in;
@@ -818,7 +856,11 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
     cudaMemsetAsync(row_slot, 0xff, (size_t)mpad * 4, st);
   }
 #undef LEWI_ROUTE_ER
-  const RouteRankArgs ra{t, logits ? topk_idx : flat_in, chunk_hist, ca.chunk_probs, n_chunks, chunk_slots};
+  if (scanned) {
+    route_scan_kernel<<<(E + kWarp - 1) / kWarp, kScanThreads, 0, st>>>(chunk_hist, n_chunks, E);
+    LEWI_CHECK_LAUNCH();
+  }
+  const RouteRankArgs ra{t, logits ? topk_idx : flat_in, chunk_hist, ca.chunk_probs, n_chunks, chunk_slots, scanned};
   static bool done[64] = {false};
   // s_run [kRouteWarps][E] also holds one partial probability sum per thread
   const size_t smem = ((size_t)chunk_slots + (size_t)(kRouteWarps * E > kRouteThreads ? kRouteWarps * E : kRouteThreads)) * 4;

@@ -220,3 +220,25 @@ def test_first_call_of_a_process_with_nearly_48_kb_of_shared_memory(cuda, t, e, 
   code = f"import sys; sys.path[:0] = [{os.path.dirname(here)!r}, {here!r}]; import test_gpu_routing as r; r.route_once({t}, {e}, {k})"
   res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
   assert res.returncode == 0, res.stderr[-2000:]
+
+
+@pytest.mark.parametrize("t,e,k", [(2_802_000, 8, 6), (17_500_003, 37, 0), (14_000_000, 500, 0)])
+def test_more_chunks_than_a_cta_adds_up_itself(cuda, t, e, k):
+  """Beyond 512 chunks (14.5 million slots on 148 SMs) a scan of the chunks' histograms comes in between; 14 million are just
+  below.  Against a stable sort; the probability sums are float32 sums of t terms in [0, 1], in parts."""
+  from lewi_surge_b200 import layer, ops
+  gen = torch.Generator(device=cuda).manual_seed(t + e)
+  if k:
+    logits = torch.randn(t, e, generator=gen, device=cuda)
+    tb = layer.router_topk(logits, k)
+    flat, order, pos = tb.topk_idx.reshape(-1), tb.order, tb.pos
+    assert torch.equal(torch.sort(torch.topk(logits, k, dim=1).indices, dim=1).values.int(), torch.sort(tb.topk_idx, dim=1).values)
+    want = torch.softmax(logits.double(), 1).sum(0)
+    assert float(((tb.probs_sum.double() - want).abs() / want).max()) <= 1e-5
+    assert torch.equal(tb.row_slot[tb.pad_pos.long()].long(), torch.arange(t * k, device=cuda))
+  else:
+    flat = torch.randint(0, e, (t,), generator=gen, device=cuda, dtype=torch.int32)
+    order, pos = ops.sort_indices(flat, e)
+  want = torch.sort(flat, stable=True).indices
+  assert torch.equal(order.long(), want)
+  assert torch.equal(pos.long()[want], torch.arange(flat.numel(), device=cuda))
