@@ -1,7 +1,7 @@
 // Router post-processing and the stable counting sort of routed slots.
 //
 // No atomics whose order could show, so every integer output is reproducible:
-//   up to kFusedTokens tokens   route_fused_kernel: one CTA does everything;
+//   a handful of tokens         route_fused_kernel: one CTA does everything (route_fused() says up to where);
 //   otherwise                   route_chunk_kernel: one CTA per chunk of slots ((soft-max + top-k + renormalise when fed
 //                               logits) and a histogram of the chunk's expert ids), then route_rank_kernel: every CTA adds
 //                               up the histograms of all chunks (one chunk per SM up to 4.8 million slots, so that is a few loads
@@ -19,7 +19,6 @@ namespace lewi {
 
 constexpr int kRouteThreads = 512;
 constexpr int kRouteWarps = kRouteThreads / kWarp;
-constexpr int kFusedTokens = 128;       // one CTA routes up to this many tokens (two rounds of 16 warps x 4 tokens)
 constexpr int kMinChunkSlots = 128;     // lewi_route_workspace_bytes counts on it
 constexpr int kMaxChunkSlots = 32768;   // a chunk's expert ids and 17 rows of 512 counters fit in 200 KB of shared memory
 constexpr int kScanChunks = 512;        // see route_scan_kernel
@@ -145,6 +144,16 @@ __device__ __forceinline__ void warp_softmax_topk(const float* const (&rows)[NT]
 
 // tokens a warp works on at once: fewer when a lane holds many experts
 template <int ER> struct RouteGroup { static constexpr int NT = ER <= 4 ? 4 : (ER <= 8 ? 2 : 1); };
+
+// Whether one CTA routes the whole call: while its warps take their tokens in one round, or where there is one chunk of slots anyway
+// (and its experts do not make the kernel spill).  A second round doubles the time, two launches spread the tokens over the SMs.
+// One CTA and two launches, in us: 128 experts top-6 8 tokens 9.1 and 12.1, 64 12.7 and 12.8, 128 20.6 and 13.0; 256 top-8 32 12.8 and
+// 13.8, 64 19.4 and 13.5; 512 top-8 16 16.3 and 18.1, 32 23.0 and 15.6; top-1 128 tokens (one chunk): 64 experts 10.6 and
+// 13.1, 256 18.3 and 21.5, 512 38.7 and 32.0.
+inline bool route_fused(long long tokens, int E, int n_chunks) {
+  const int round = kRouteWarps * (E <= 128 ? RouteGroup<4>::NT : (E <= 256 ? RouteGroup<8>::NT : RouteGroup<16>::NT));
+  return tokens > 0 && (tokens <= round || (n_chunks == 1 && E <= 256));
+}
 
 struct RouteChunkArgs {
   const float* logits;        // [T,E] or null
@@ -826,7 +835,7 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
   const bool scanned = n_chunks > kScanChunks;
   const long long hist_rows = n_chunks + (scanned ? 1 : 0), need = (hist_rows + n_chunks) * E * 4;
   if (ws == nullptr || ws_bytes < need) return LEWI_ERR_WORKSPACE;   // also where the one-CTA path would not touch it
-  if (logits != nullptr && T > 0 && T <= kFusedTokens) {
+  if (logits != nullptr && route_fused(T, E, n_chunks)) {
     const RouteFusedArgs fa{t, logits, topk_idx, topk_w, mpad, k};
     LEWI_ROUTE_ER(launch_route_fused<ER>(st, fa));
     return LEWI_OK;

@@ -41,10 +41,11 @@ def test_router_topk_bit_exact(cuda, t, e, k):
   check_tables(tb, logits, k, e)
 
 
-@pytest.mark.parametrize("t,e,k", [(128, 16, 6), (129, 16, 1), (2400, 8, 2), (127, 200, 3), (20000, 40, 4), (500, 512, 1)])
+@pytest.mark.parametrize("t,e,k", [(128, 16, 6), (129, 16, 1), (2400, 8, 2), (127, 200, 3), (20000, 40, 4), (500, 512, 1), (64, 128, 6),
+                                   (65, 128, 6), (32, 256, 8), (33, 256, 8), (16, 512, 8), (17, 512, 8), (100, 256, 1)])
 def test_router_at_the_edges_of_its_two_paths(cuda, t, e, k):
-  """One CTA up to 128 tokens, chunks beyond; few experts (one partial sum per thread), an odd number, the most; and the
-  load-balance loss, a sum of e non-negative float32 terms: off by at most e * 2^-24 of it."""
+  """One CTA for one round of tokens (64, 32 or 16 by the experts) or one chunk, several beyond; few experts (one partial sum per
+  thread), an odd number, the most; and the load-balance loss, a sum of e non-negative float32 terms: off by at most e * 2^-24 of it."""
   from lewi_surge_b200 import layer
   logits = np.random.default_rng(t + e).standard_normal((t, e)).astype(np.float32)
   aux = torch.empty(1, dtype=torch.float32, device=cuda)
