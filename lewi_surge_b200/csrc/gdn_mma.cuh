@@ -7,7 +7,7 @@
 // tcgen05.ld -> split -> tcgen05.st and two commit waits per 64-token chunk, and 128 state columns per CTA: 64 CTAs at
 // batch 8 x 8 heads.)
 //
-// Float32 operands are cut into three bf16 pieces (8 + 8 + 8 mantissa bits, nothing of the 24 is lost), so a product of a
+// Float32 operands are cut into three bf16 pieces (8 + 8 + 8 mantissa bits, see split3 for what that excludes), so a product of a
 // float32 and a bf16 operand is three MMAs and one of two float32 operands six (piece products below 2^-24 of the whole
 // are left out); all of them accumulate in float32, which the tensor core truncates (see Prod2).  Measured on a B200: one
 // m16n8k16 per 8 cycles and scheduler.
@@ -198,7 +198,8 @@ __device__ __forceinline__ void mma2_x6(float (&d0)[4], float (&d1)[4], const Fr
   x.add_to(d0, d1);
 }
 
-// two floats -> three packed bf16 pairs, x = p0 + p1 + p2 exactly (up to float32 subnormals)
+// two floats -> three packed bf16 pairs, x = p0 + p1 + p2 exactly for |x| below bf16's largest value (3.39e38), down to float32
+// subnormals.  Larger values, infinities and NaN have NaN among their pieces: what is infinite comes out of a product as NaN.
 __device__ __forceinline__ void split3(float x0, float x1, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
   p0 = pack_bf16(x0, x1);
   x0 -= bf16_lo(p0);

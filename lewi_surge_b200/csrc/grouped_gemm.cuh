@@ -653,7 +653,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           }
         }
       } else if constexpr (EPI == SWIGLU) {
-        // h [rows, f] through tm_c, gu [rows][2][f] through tm_d; this warp owns 64 h columns: three 4 KB tiles
+        // h [rows, f] through tm_c, gu [rows][2][f] through tm_d; this warp owns 64 columns of g, u and h
         const int f = a.N;
         const int n64 = t.n0 + col_half * 64;
         if (rows_valid > 0 && n64 < n_end) {

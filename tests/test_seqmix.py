@@ -271,11 +271,14 @@ def test_oracle_backward_without_a_state_matches_autograd():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("b,s,h,kd,vd", [(1, 1, 1, 8, 8), (1, 129, 2, 128, 512), (13, 70, 2, 72, 128), (2, 65, 13, 24, 120), (10, 127, 8, 104, 128),
-                                         (10, 63, 8, 56, 104)])
+                                         (10, 63, 8, 56, 104), (8, 130, 8, 128, 128), (16, 70, 8, 64, 64), (2, 130, 8, 128, 128), (2, 70, 8, 64, 128),
+                                         (10, 70, 8, 64, 16), (10, 65, 8, 72, 16)])
 def test_gdn_kernels_for_every_split_of_the_scan(cuda, b, s, h, kd, vd):
-  """One, two and eight groups of 16 state columns per scan CTA (four is covered above), one and two 64-column tiles of the
-  state's rows, head dimensions that fill no tile, one token, a full chunk and one token more or less.  Against the oracle:
-  bf16 results within a few roundings, the float32 gradients of g and the state 2e-3 as above."""
+  """One, two, four and eight groups of 16 state columns per scan CTA, one and two 64-column tiles of the state's rows, head dimensions
+  that fill no tile, one token, a full chunk and one token more or less.  The two scans of the backward pass on 148 SMs: in one launch
+  with one group (the first shape) or with two where one would not fit ((2, 130, ..) and (2, 70, ..)), in two with one group
+  (the last two shapes), two (13, 70, ..), four ((8, 130, ..) and (16, 70, ..)) and eight ((10, 127, ..) and (10, 63, ..)).
+  Against the oracle: bf16 results within a few roundings, the float32 gradients of g and the state 2e-3 as above."""
   from lewi_surge_b200 import seqmix, _lib
   i = _gdn_inputs(b, s, h, kd, vd, seed=s + vd)
   names = ("q", "k", "v", "g", "beta", "h0")
@@ -369,3 +372,25 @@ def test_gdn_takes_outputs_and_upstream_gradients_at_any_address(cuda, b, s, h, 
 
   for shift in (1, 2):
     assert all(torch.equal(x, y) for x, y in zip(run(0), run(shift)))
+
+
+@pytest.mark.gpu
+def test_gdn_values_that_are_not_finite_stay_in_their_column(cuda):
+  """An infinite v reaches its own column of V only, from its block of 16 tokens on (the reference's masked products reach the whole
+  chunk); an infinite state its own column only; neither turns finite.  Everything else keeps its bits."""
+  from lewi_surge_b200 import seqmix
+  b, s, h, d = 1, 200, 2, 64
+  i = _gdn_inputs(b, s, h, d, d, seed=21)
+  names = ("q", "k", "v", "g", "beta", "h0")
+  t = {n: to_dev(i[n], torch.float32 if n in ("g", "h0") else torch.bfloat16, cuda) for n in names}
+  run = lambda **new: seqmix.chunk_gated_delta_rule(*({**t, **new}[n] for n in names[:5]), initial_state={**t, **new}["h0"])
+  want_o, want_h = run()
+  v, h0 = t["v"].clone(), t["h0"].clone()
+  v[0, 100, 0, 5] = float("inf")   # the 37th token of the second chunk: its block begins at token 96
+  h0[0, 1, 3, 7] = float("inf")
+  for (o, hf), head, col, first, sure in ((run(v=v), 0, 5, 96, 100), (run(h0=h0), 1, 7, 0, 0)):
+    keep_o, keep_h = torch.ones_like(o, dtype=torch.bool), torch.ones_like(hf, dtype=torch.bool)
+    keep_o[:, first:, head, col] = False
+    keep_h[:, head, :, col] = False
+    assert torch.equal(o[keep_o], want_o[keep_o]) and torch.equal(hf[keep_h], want_h[keep_h])
+    assert not torch.isfinite(o[0, sure:, head, col]).any() and not torch.isfinite(hf[0, head, :, col]).any()
