@@ -206,7 +206,7 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint4 v) {
 }
 
 // One CTA per chunk and head, two CTAs per SM.  About 1,300 MMAs per chunk (triangular blocks are skipped) and some 100 KB
-// in and out.  Latency-bound (ncu: 0.37 of the issue slots, no pipe above 0.4).  B=8, S=4096, H=8, K=V=128: 0.225 ms (0.79 ms
+// in and out.  Latency-bound (ncu: 0.38 of the issue slots, tensor pipe 0.21).  B=8, S=4096, H=8, K=V=128: 0.225 ms (0.79 ms
 // with the products in float32 on the CUDA cores).
 template <int KB>
 __global__ void __launch_bounds__(kChunkThreads, 2)
@@ -486,7 +486,7 @@ struct ScanArgs {
 // q products while the others arrive, and add all parts in the same order; each finishes 64/KS tokens of o.
 // 696 m16n8k16 per group and chunk (K = 128), 5,600 cycles of one scheduler at the measured 8 cycles each; a single warp per
 // scheduler reached 9,500 (splitting and loading do not overlap its own MMAs), so the launch splits K until every scheduler has
-// two warps, or K is in quarters.  B=8, S=4096, H=8, K=V=128: 0.31 ms (1.61 ms in float32 on the CUDA cores), tensor pipe 65 %
+// two warps, or K is in quarters.  B=8, S=4096, H=8, K=V=128: 0.31 ms (1.61 ms in float32 on the CUDA cores), tensor pipe 66 %
 // active; B=1, S=1000: 0.035 ms (0.23 ms).
 // STATES (the first pass of the gradient): no output; the state at the start of every chunk and v_new are stored instead.
 // A producer warp keeps a ring of two chunks filled by TMA: issuing the nine copies takes a thousand cycles, which the other
