@@ -346,9 +346,10 @@ int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v
  *              workspace can serve fwd and bwd of any number of layers on the same stream.
  * Both buffers must be 16-byte aligned.  `has_gate` (layout functions) = whether w_sg will be passed.
  *
- * side_stream (may be null or equal to stream): the shared expert, which needs only x / dout, is queued there
+ * side_stream (may be null or equal to stream): the shared expert, which needs only x / dout, and the forward pass's
+ * experts of many rows beside those of few, are queued there
  * between two events so that it overlaps the memory-bound routing, dispatch and gather kernels; the call
- * returns with `stream` waiting for it.  The four events per device are created on first use and kept.
+ * returns with `stream` waiting for it.  The events per device are created on first use and kept.
  *
  * router_prepared (may be null): the bf16 pieces of w_router that the router GEMMs read, as written by
  * lewi_moe_prepare_router (lewi_moe_router_prepared_bytes(d,E) bytes); pass it to skip that conversion in
@@ -373,8 +374,8 @@ int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v
 #define LEWI_MOE_RES_POS 10         /* i32 [T*k]        */
 #define LEWI_MOE_RES_PAD_POS 11     /* i32 [T*k]        */
 #define LEWI_MOE_RES_ROW_SLOT 12    /* i32 [Mpad]       */
-#define LEWI_MOE_RES_XS 13          /* bf16 [Mpad,d]    */
-#define LEWI_MOE_RES_GU 14          /* bf16 [Mpad,2f]   */
+#define LEWI_MOE_RES_XS 13          /* bf16 [Mpad,d]; few tokens: not (all) written, bwd picks the rows from x */
+#define LEWI_MOE_RES_GU 14          /* bf16 [Mpad,2f] (rows without a slot undefined) */
 #define LEWI_MOE_RES_H 15           /* bf16 [Mpad,f] (times the router weight of the row) */
 #define LEWI_MOE_RES_GUS 16         /* bf16 [T,2fs]     */
 #define LEWI_MOE_RES_HS 17          /* bf16 [T,fs] (times the gate, if any) */

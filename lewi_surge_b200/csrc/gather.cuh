@@ -356,6 +356,31 @@ inline int gather_grid(long long rows) {
 }
 
 // smallest supported VPL in {1,2,4,8,16} covering the row, or 0
+// Padded rows of the experts that have more than one row block: row r = x[row_slot[r] / k], zeros where row_slot[r] < 0; other experts'
+// blocks are passed over.  A CTA takes 16 rows, two per warp (a block per CTA, 16 rows per warp: 15 us instead of 4 for eight experts of
+// 700 rows, and the experts' GEMMs wait for it).
+constexpr int kHeavyRows = 16;
+__global__ void __launch_bounds__(256) gather_heavy_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ row_slot,
+                                                           const int32_t* __restrict__ block_expert, const int32_t* __restrict__ n_blocks,
+                                                           const int32_t* __restrict__ counts, __nv_bfloat16* __restrict__ out, int max_blocks,
+                                                           int k, int d) {
+  constexpr int kBlockRows = 128, kParts = kBlockRows / kHeavyRows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, units = min(max_blocks, n_blocks[0]) * kParts;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    if (counts[block_expert[u / kParts]] <= kBlockRows) continue;
+    const long long row = (long long)u * kHeavyRows + warp * 2;
+    const int s0 = row_slot[row], s1 = row_slot[row + 1];
+    const __nv_bfloat16 *src0 = x + (long long)(s0 < 0 ? 0 : s0 / k) * d, *src1 = x + (long long)(s1 < 0 ? 0 : s1 / k) * d;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll 4
+    for (int c = lane * 8; c < d; c += 256) {
+      const uint4 v0 = ld_nc_v4(src0 + c), v1 = ld_nc_v4(src1 + c);
+      st_v4(out + row * d + c, s0 < 0 ? zero : v0);
+      st_v4(out + (row + 1) * d + c, s1 < 0 ? zero : v1);
+    }
+  }
+}
+
 inline int pick_vpl(int d, int elem_bytes) {
   const long long row_bytes = (long long)d * elem_bytes;
   if (row_bytes % 16 != 0) return 0;

@@ -86,6 +86,7 @@ struct Args {
   const float* col_bias;        // PLAIN: optional f32 per output column
   const float* r1_row;          // PLAIN: optional rank-one term added to the product: out[r,n] += r1_row[r] * r1_col[n]
   const float* r1_col;
+  int skip_rows;                // pair kernels, NN / NT: experts of at most this many padded rows are left out
   int tn_part_rows;             // TN over several experts: > 0 cuts an expert's contraction into parts of this many rows
                                 // (a multiple of 64); experts with more than one part go through `partial`
   const int32_t* scale_idx;     // SWIGLU / DSWIGLU: padded row -> index into scale_src (negative: scale 0; null: the row itself)
@@ -366,7 +367,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return max(1, (rows_e + a.tn_part_rows - 1) / a.tn_part_rows); });
   } else if constexpr (PAIR) {
     // exclusive prefix of ceil(blocks_e / 2)
-    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [](int rows_e) { return (rows_e / BM + 1) >> 1; });
+    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return rows_e > a.skip_rows ? (rows_e / BM + 1) >> 1 : 0; });
   }
   if (warp == 1) {
     if constexpr (PAIR) {
@@ -563,6 +564,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
       // What the epilogue needs per row besides the accumulator is fetched now, while the tensor cores still work on
       // the tile: the row's scale (a dependent pair of loads under SWIGLU / DSWIGLU), rank-one factor or destination.
       [[maybe_unused]] float row_sc = 1.0f, row_r1 = 0.f;
+      [[maybe_unused]] bool no_slot = false;   // a padding row: what g|u holds there is not defined
       [[maybe_unused]] unsigned long long my_dst = 0;
       if (lane < rows_valid) {
         if constexpr (EPI == PLAIN) {
@@ -572,6 +574,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
           if (a.scale_src != nullptr) {
             const long long gi = a.scale_idx != nullptr ? (long long)a.scale_idx[wrow0 + lane] : wrow0 + lane;
             row_sc = gi >= 0 ? a.scale_src[gi] : 0.f;
+            no_slot = gi < 0;
           }
         } else if constexpr (EPI == SCATTER) {
           const int code = a.ret[wrow0 + lane];
@@ -729,6 +732,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
               g[q * 8 + 4] = bf16_lo(pg.z); g[q * 8 + 5] = bf16_hi(pg.z); g[q * 8 + 6] = bf16_lo(pg.w); g[q * 8 + 7] = bf16_hi(pg.w);
               u[q * 8 + 0] = bf16_lo(pu.x); u[q * 8 + 1] = bf16_hi(pu.x); u[q * 8 + 2] = bf16_lo(pu.y); u[q * 8 + 3] = bf16_hi(pu.y);
               u[q * 8 + 4] = bf16_lo(pu.z); u[q * 8 + 5] = bf16_hi(pu.z); u[q * 8 + 6] = bf16_lo(pu.w); u[q * 8 + 7] = bf16_hi(pu.w);
+            }
+            if (no_slot) {
+#pragma unroll
+              for (int q = 0; q < 32; ++q) g[q] = u[q] = 0.f;
             }
             uint32_t r[32];
             if (has_acc) {

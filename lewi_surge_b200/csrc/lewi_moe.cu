@@ -3,6 +3,7 @@
 #include "ep.cuh"
 #include "ep_unique.cuh"
 #include "gather.cuh"
+#include "few_gemm.cuh"
 #include "grouped_gemm.cuh"
 #include "moe_layer.cuh"
 #include "router_gemm.cuh"
@@ -336,6 +337,7 @@ struct RowGroupArgs {
   const int32_t* pad_offsets;
   int64_t rows;
   int E;
+  int skip_rows = 0;   // pair kernels: experts of at most this many padded rows are left out
 };
 
 // The CTA-pair kernels derive a row block's expert from pad_offsets; the single-CTA ones read
@@ -383,6 +385,7 @@ inline void fill_common(gg::Args& a, const RowGroupArgs& r) {
   a.col_bias = nullptr;
   a.r1_row = nullptr;
   a.r1_col = nullptr;
+  a.skip_rows = r.skip_rows;
   a.tn_part_rows = 0;
   a.scale_src = nullptr;
   a.scale_idx = nullptr;
@@ -413,9 +416,104 @@ int64_t lewi_router_logits_workspace_bytes(int d, int E) {
 }
 
 namespace {
+// One group of `rows` rows over `cols`-wide tiles: rows per unit, the fewest (in powers of two of 16) whose tiles one wave holds.
+inline int few_unit_rows(int64_t rows, int n_tiles) {
+  int u = 16;
+  while (u < few::MAX_ROWS && (rows + u - 1) / u * n_tiles > num_sms()) u *= 2;
+  return u;
+}
+inline void few_one_group(few::Args& a, int64_t rows, int unit_rows) {
+  a.rows = rows;
+  a.unit_rows = unit_rows;
+  a.units = (int)((rows + unit_rows - 1) / unit_rows);
+  a.E = 1;
+}
+// The router's projection: as long as one wave holds its tiles of 128 rows.  Forward pass with the pair kernel -> so (no shared expert,
+// routed experts on the pair kernels): d 1024, 128 experts, 512 tokens 162 -> 152 us, 4096 tokens 188 -> 182; d 2048, 256 experts, 512
+// tokens 541 -> 524, 4096 tokens (128 tiles) 641 -> 637, 8192 tokens (256 tiles) 924 -> 932.
+inline bool few_router(int64_t T, int E) { return (T + 127) / 128 * ((E + 63) / 64) <= num_sms(); }
+// The shared expert's projections run beside the router and the routing, on the SMs these leave; where they are no longer hidden behind
+// them the pair kernels' tiles are better: d 1024, width 512: 8 tokens 86 -> 78 us a forward pass, 64 tokens 125 -> 123, 200 tokens
+// 125 -> 127, 700 tokens 129 -> 135; d 2048, width 2048: 32 tokens 301 -> 293, 64 tokens 375 -> 375, 128 tokens 422 -> 430.
+inline bool few_shared(int64_t T) { return T <= 64; }
+
+int few_logits(cudaStream_t st, const void* x, const void* w3, const float* bias, float* logits, int64_t T, int d, int E) {
+  few::Args a = {};
+  const int u = few_unit_rows(T, (E + 63) / 64);
+  few_one_group(a, T, u);
+  a.kb_total = 3 * d / few::BK;
+  a.k_wrap = d;
+  a.N = E;
+  a.out = logits;
+  a.col_bias = bias;
+  CUtensorMap tw, tr;
+  if (!gg::make_map(&tw, w3, (uint64_t)E, (uint64_t)3 * d, 1, 64, 64) || !gg::make_map(&tr, x, (uint64_t)d, (uint64_t)T, 0, 64, 16)) return LEWI_ERR_CUDA;
+  return few::launch<few::LOGITS>(st, tw, tw, tr, a, u);
+}
+
+// Row blocks of the routing tables (null block_expert: one group of `rows` rows).
+struct FewGroups {
+  const int32_t *block_expert, *n_blocks, *pad_offsets, *counts;
+  int max_group;     // experts of more rows are left out
+  int64_t rows;      // rows of the row-indexed tensors
+  int64_t max_rows;  // most rows that a group can have
+  int E;
+};
+inline int few_groups(few::Args& a, const FewGroups& r, int n_tiles) {
+  if (r.block_expert == nullptr) {
+    const int u = few_unit_rows(r.rows, n_tiles);
+    few_one_group(a, r.rows, u);
+    return u;
+  }
+  a.block_expert = r.block_expert;
+  a.n_blocks = r.n_blocks;
+  a.pad_offsets = r.pad_offsets;
+  a.counts = r.counts;
+  a.max_group = r.max_group;
+  a.E = r.E;
+  a.units = (int)(r.rows / few::MAX_ROWS);
+  return (int)(r.max_rows < few::MAX_ROWS ? r.max_rows : few::MAX_ROWS);
+}
+
+// h = SwiGLU(x_rows . wg, x_rows . wu) * scale, gu = both products; the rows of x are those of the blocks, or picked by row_slot[r] / k.
+int few_gateup(void* stream, const void* x, int64_t x_rows, const int32_t* row_slot, int k, const int32_t* scale_idx, const float* scale_src,
+               const void* wg, const void* wu, void* gu, void* h, const FewGroups& r, int d, int f) {
+  if (!aligned16(x) || !aligned16(wg) || !aligned16(wu) || !aligned16(gu) || !aligned16(h) || d % 8 != 0 || f % 8 != 0) return LEWI_ERR_SHAPE;
+  few::Args a = {};
+  const int max_rows = few_groups(a, r, (f + 63) / 64);
+  a.gather_idx = row_slot;
+  a.gather_div = k;
+  a.x = reinterpret_cast<const __nv_bfloat16*>(x);
+  a.K = d;
+  a.kb_total = (d + few::BK - 1) / few::BK;
+  a.N = f;
+  a.out = h;
+  a.gu = reinterpret_cast<__nv_bfloat16*>(gu);
+  a.scale_idx = scale_idx;
+  a.scale_src = scale_src;
+  CUtensorMap tg, tu, tr;
+  if (!gg::make_map(&tg, wg, (uint64_t)f, (uint64_t)d, (uint64_t)r.E, 64, 64) || !gg::make_map(&tu, wu, (uint64_t)f, (uint64_t)d, (uint64_t)r.E, 64, 64) ||
+      !gg::make_map(&tr, x, (uint64_t)d, (uint64_t)x_rows, 0, 64, 16))
+    return LEWI_ERR_CUDA;
+  return few::launch<few::SWIGLU>(as_stream(stream), tg, tu, tr, a, max_rows);
+}
+int few_down(void* stream, const void* h, const void* w, void* out, const FewGroups& r, int K, int N) {
+  if (!aligned16(h) || !aligned16(w) || !aligned16(out) || K % 8 != 0 || N % 8 != 0) return LEWI_ERR_SHAPE;
+  few::Args a = {};
+  const int max_rows = few_groups(a, r, (N + 127) / 128);
+  a.kb_total = (K + few::BK - 1) / few::BK;
+  a.N = N;
+  a.out = out;
+  CUtensorMap tw, tr;
+  if (!gg::make_map(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)r.E, 64, 64) || !gg::make_map(&tr, h, (uint64_t)K, (uint64_t)r.rows, 0, 64, 16))
+    return LEWI_ERR_CUDA;
+  return few::launch<few::PLAIN>(as_stream(stream), tw, tw, tr, a, max_rows);
+}
+
 // logits = [x x x] . [hi; mid; lo] on the tensor cores; w3 holds the three bf16 pieces of the f32 weight.
 int router_logits_tensor(cudaStream_t st, const void* x, const void* w3, const float* bias, float* logits, int64_t T,
                          int d, int E) {
+  if (few_router(T, E)) return few_logits(st, x, w3, bias, logits, T, d, E);
   CUtensorMap ta, tb;
   if (!gg::make_map(&ta, x, (uint64_t)d, (uint64_t)T, 0, 64, 128)) return LEWI_ERR_CUDA;
   if (!gg::make_map(&tb, w3, (uint64_t)E, (uint64_t)3 * d, 1, 64, 64)) return LEWI_ERR_CUDA;
@@ -492,7 +590,7 @@ inline int fill_return(gg::Args& a, const ReturnTable& rt, int row_elems) {
 
 int grouped_gemm_nn_impl(void* stream, const void* a_ptr, const void* b_ptr, void* out, const float* row_scale,
                          const int32_t* block_expert, const int32_t* n_blocks, const int32_t* pad_offsets, int64_t rows,
-                         int K, int N, int E, int out_dtype, const ReturnTable* rt);
+                         int K, int N, int E, int out_dtype, const ReturnTable* rt, int skip_rows = 0);
 }  // namespace
 
 int lewi_grouped_gemm_nn(void* stream, const void* a_ptr, const void* b_ptr, void* out, const float* row_scale,
@@ -514,10 +612,10 @@ int lewi_grouped_gemm_nn_return(void* stream, const void* a_ptr, const void* b_p
 namespace {
 int grouped_gemm_nn_impl(void* stream, const void* a_ptr, const void* b_ptr, void* out, const float* row_scale,
                          const int32_t* block_expert, const int32_t* n_blocks, const int32_t* pad_offsets, int64_t rows,
-                         int K, int N, int E, int out_dtype, const ReturnTable* rt) {
+                         int K, int N, int E, int out_dtype, const ReturnTable* rt, int skip_rows) {
   if (!a_ptr || !b_ptr || (!out && !rt) || K <= 0 || N <= 0) return LEWI_ERR_ARG;
   if (out_dtype != LEWI_BF16 && out_dtype != LEWI_F32) return LEWI_ERR_ARG;
-  RowGroupArgs r{block_expert, n_blocks, pad_offsets, rows, E};
+  RowGroupArgs r{block_expert, n_blocks, pad_offsets, rows, E, skip_rows};
   const bool pair = use_pair(r);
   if (int rc = check_rows(r)) return rc;
   if (K % 8 != 0 || N % 8 != 0 || !aligned16(a_ptr) || !aligned16(b_ptr) || !aligned16(out)) return LEWI_ERR_SHAPE;
@@ -689,12 +787,12 @@ int lewi_grouped_gemm_gateup_swiglu(void* stream, const void* xs, const void* w_
                                                 pad_offsets, rows, d, f, E);
 }
 
-int lewi_grouped_gemm_gateup_swiglu_scaled(void* stream, const void* xs, const int32_t* scale_idx,
-                                           const float* h_scale_src, const void* w_gate, const void* w_up, void* gu,
-                                           void* h, const int32_t* block_expert, const int32_t* n_blocks,
-                                           const int32_t* pad_offsets, int64_t rows, int d, int f, int E) {
+namespace {
+int gateup_swiglu_impl(void* stream, const void* xs, const int32_t* scale_idx, const float* h_scale_src, const void* w_gate, const void* w_up,
+                       void* gu, void* h, const int32_t* block_expert, const int32_t* n_blocks, const int32_t* pad_offsets, int64_t rows,
+                       int d, int f, int E, int skip_rows) {
   if (!xs || !w_gate || !w_up || !h || d <= 0 || f <= 0) return LEWI_ERR_ARG;
-  RowGroupArgs r{block_expert, n_blocks, pad_offsets, rows, E};
+  RowGroupArgs r{block_expert, n_blocks, pad_offsets, rows, E, skip_rows};
   if (int rc = check_rows(r)) return rc;
   const bool pair = use_pair(r);
   if (d % 8 != 0 || f % 8 != 0 || !aligned16(xs) || !aligned16(w_gate) || !aligned16(w_up) || !aligned16(gu) ||
@@ -719,6 +817,14 @@ int lewi_grouped_gemm_gateup_swiglu_scaled(void* stream, const void* xs, const i
   if (gu != nullptr && !gg::make_map(&tgu, gu, (uint64_t)f, 2, (uint64_t)rows, 64, 1, 32)) return LEWI_ERR_CUDA;
   const long long tiles = (long long)a.n_blocks_host * ((f + gg::BN / 2 - 1) / (gg::BN / 2));
   return gg::launch_auto<gg::NN, gg::SWIGLU>(pair, as_stream(stream), ta, tb, tb2, a, tiles, &th, gu ? &tgu : &th);
+}
+}  // namespace
+
+int lewi_grouped_gemm_gateup_swiglu_scaled(void* stream, const void* xs, const int32_t* scale_idx,
+                                           const float* h_scale_src, const void* w_gate, const void* w_up, void* gu,
+                                           void* h, const int32_t* block_expert, const int32_t* n_blocks,
+                                           const int32_t* pad_offsets, int64_t rows, int d, int f, int E) {
+  return gateup_swiglu_impl(stream, xs, scale_idx, h_scale_src, w_gate, w_up, gu, h, block_expert, n_blocks, pad_offsets, rows, d, f, E, 0);
 }
 
 int lewi_grouped_gemm_dh_dswiglu(void* stream, const void* dys, const void* w_down, const void* gu, void* dgu,
@@ -1321,7 +1427,9 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
   auto res = [&](int i) { return R + ro[i]; };
   cudaStream_t st = as_stream(stream), sd = as_stream(side_stream);
   const bool shared = fs > 0;
-  const bool fork = shared && side_stream != nullptr && side_stream != stream;
+  // few rows per expert: the kernels of few_gemm.cuh; with more than a few blocks' worth of tokens only for experts of one block
+  const bool heavy = T > moe::kFewTokens, few = moe::few_routed(T, D.M, E) && (!heavy || gg::pair_mode());
+  const bool fork = (shared || (few && heavy)) && side_stream != nullptr && side_stream != stream;
   moe::Events* ev = fork ? moe::events() : nullptr;
   if (fork && ev == nullptr) return LEWI_ERR_CUDA;
   void* sh_stream = fork ? side_stream : stream;
@@ -1351,6 +1459,14 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
       moe::mark("shared_gate", sh_stream);
     }
     // with a gate, hs (and so the shared output) is stored already multiplied by it
+    if (few_shared(T)) {
+      const FewGroups one{nullptr, nullptr, nullptr, nullptr, 0, T, T, 1};
+      LEWI_TRY(few_gateup(sh_stream, x, T, nullptr, 1, nullptr, gate, ws_gate, ws_up, res(LEWI_MOE_RES_GUS), res(LEWI_MOE_RES_HS), one, d, fs));
+      moe::mark("shared_gateup_swiglu", sh_stream);
+      LEWI_TRY(few_down(sh_stream, res(LEWI_MOE_RES_HS), ws_down, ysh, one, fs, d));
+      moe::mark("shared_down", sh_stream);
+      return LEWI_OK;
+    }
     LEWI_TRY(lewi_grouped_gemm_gateup_swiglu_scaled(sh_stream, x, nullptr, gate, ws_gate, ws_up, res(LEWI_MOE_RES_GUS),
                                                     res(LEWI_MOE_RES_HS), nullptr, nullptr, nullptr, T, d, fs, 1));
     moe::mark("shared_gateup_swiglu", sh_stream);
@@ -1385,20 +1501,46 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
                             lewi_route_workspace_bytes(D.M, E)));
   moe::mark("router_topk", stream);
   }
-  {
-  // dispatch: padded row r holds token row_slot[r] / k (zero row where row_slot[r] < 0), written in token order
-  moe::Range nvtx_dispatch("moe_permute_dispatch");
-  LEWI_TRY(lewi_dispatch_rows(stream, x, pad_pos, row_slot, res(LEWI_MOE_RES_XS), T, k, d, D.Mpad, n_blocks, moe::kBlock));
-  moe::mark("dispatch_gather", stream);
-  }
   // h carries the router weight of its row, so the down projection yields weighted outputs
-  LEWI_TRY(lewi_grouped_gemm_gateup_swiglu_scaled(stream, res(LEWI_MOE_RES_XS), row_slot, topk_w, w_gate, w_up,
-                                                  res(LEWI_MOE_RES_GU), res(LEWI_MOE_RES_H), block_expert, n_blocks,
-                                                  pad_offsets, D.Mpad, d, f, E));
-  moe::mark("gemm_gateup_swiglu", stream);
-  LEWI_TRY(lewi_grouped_gemm_nn(stream, res(LEWI_MOE_RES_H), w_down, Wk + W.ys, nullptr, block_expert, n_blocks,
-                                pad_offsets, D.Mpad, f, d, E, LEWI_BF16));
-  moe::mark("gemm_down", stream);
+  if (few) {
+    const int32_t* counts = reinterpret_cast<const int32_t*>(res(LEWI_MOE_RES_COUNTS));
+    if (heavy) {   // experts of several blocks go through the pair kernels, beside the others where there is a side stream
+      if (fork && (cudaEventRecord(ev->routed_fwd, st) != cudaSuccess || cudaStreamWaitEvent(sd, ev->routed_fwd, 0) != cudaSuccess))
+        return LEWI_ERR_CUDA;
+      const int max_blocks = (int)(D.Mpad / moe::kBlock);
+      const int units = max_blocks * (moe::kBlock / kHeavyRows);
+      gather_heavy_kernel<<<units < 4 * num_sms() ? units : 4 * num_sms(), 256, 0, as_stream(sh_stream)>>>(
+          reinterpret_cast<const __nv_bfloat16*>(x), row_slot, block_expert, n_blocks, counts,
+          reinterpret_cast<__nv_bfloat16*>(res(LEWI_MOE_RES_XS)), max_blocks, k, d);
+      LEWI_CHECK_LAUNCH();
+      moe::mark("dispatch_gather", sh_stream);
+      LEWI_TRY(gateup_swiglu_impl(sh_stream, res(LEWI_MOE_RES_XS), row_slot, topk_w, w_gate, w_up, res(LEWI_MOE_RES_GU), res(LEWI_MOE_RES_H),
+                                  block_expert, n_blocks, pad_offsets, D.Mpad, d, f, E, moe::kBlock));
+      moe::mark("gemm_gateup_swiglu_heavy", sh_stream);
+      LEWI_TRY(grouped_gemm_nn_impl(sh_stream, res(LEWI_MOE_RES_H), w_down, Wk + W.ys, nullptr, block_expert, n_blocks, pad_offsets, D.Mpad,
+                                    f, d, E, LEWI_BF16, nullptr, moe::kBlock));
+      moe::mark("gemm_down_heavy", sh_stream);
+    }
+    const FewGroups blocks{block_expert, n_blocks, pad_offsets, counts, heavy ? moe::kBlock : 0x7fffffff, D.Mpad, T, E};
+    LEWI_TRY(few_gateup(stream, x, T, row_slot, k, row_slot, topk_w, w_gate, w_up, res(LEWI_MOE_RES_GU), res(LEWI_MOE_RES_H), blocks, d, f));
+    moe::mark("gemm_gateup_swiglu", stream);
+    LEWI_TRY(few_down(stream, res(LEWI_MOE_RES_H), w_down, Wk + W.ys, blocks, f, d));
+    moe::mark("gemm_down", stream);
+  } else {
+    {
+    // dispatch: padded row r holds token row_slot[r] / k (zero row where row_slot[r] < 0), written in token order
+    moe::Range nvtx_dispatch("moe_permute_dispatch");
+    LEWI_TRY(lewi_dispatch_rows(stream, x, pad_pos, row_slot, res(LEWI_MOE_RES_XS), T, k, d, D.Mpad, n_blocks, moe::kBlock));
+    moe::mark("dispatch_gather", stream);
+    }
+    LEWI_TRY(lewi_grouped_gemm_gateup_swiglu_scaled(stream, res(LEWI_MOE_RES_XS), row_slot, topk_w, w_gate, w_up,
+                                                    res(LEWI_MOE_RES_GU), res(LEWI_MOE_RES_H), block_expert, n_blocks,
+                                                    pad_offsets, D.Mpad, d, f, E));
+    moe::mark("gemm_gateup_swiglu", stream);
+    LEWI_TRY(lewi_grouped_gemm_nn(stream, res(LEWI_MOE_RES_H), w_down, Wk + W.ys, nullptr, block_expert, n_blocks,
+                                  pad_offsets, D.Mpad, f, d, E, LEWI_BF16));
+    moe::mark("gemm_down", stream);
+  }
   if (shared && !fork) LEWI_TRY(shared_fwd());
   if (fork) {
     if (cudaEventRecord(ev->join_fwd, sd) != cudaSuccess || cudaStreamWaitEvent(st, ev->join_fwd, 0) != cudaSuccess)
@@ -1550,7 +1692,14 @@ int lewi_moe_bwd(void* stream, void* side_stream, const void* dout, const void* 
   LEWI_TRY(lewi_grouped_gemm_dx(stream, Wk + W.dgu, w_gate, w_up, Wk + W.dxs, block_expert, n_blocks, pad_offsets, D.Mpad,
                                 d, f, E));
   moe::mark("gemm_dx", stream);
-  LEWI_TRY(lewi_grouped_gemm_tn(stream, res(LEWI_MOE_RES_XS), Wk + W.dgu, dw_gate, dw_up, pad_offsets, D.Mpad, d, 2 * f, E,
+  // (the forward pass of few rows picks them from x as it goes: its rows in padded order are written here)
+  const void* xs = res(LEWI_MOE_RES_XS);
+  if (moe::few_routed(T, D.M, E)) {
+    LEWI_TRY(lewi_dispatch_rows(stream, x, pad_pos, row_slot, Wk + W.xs, T, k, d, D.Mpad, n_blocks, moe::kBlock));
+    moe::mark("dispatch_gather", stream);
+    xs = Wk + W.xs;
+  }
+  LEWI_TRY(lewi_grouped_gemm_tn(stream, xs, Wk + W.dgu, dw_gate, dw_up, pad_offsets, D.Mpad, d, 2 * f, E,
                                 wgrad_dtype, W.tn_e_bytes > 0 ? Wk + W.tn_e : nullptr, W.tn_e_bytes));
   moe::mark("gemm_dw_gateup", stream);
   if (!fork) {

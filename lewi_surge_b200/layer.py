@@ -56,7 +56,8 @@ def _mark(name):
 
 
 # The shared expert depends only on x (forward) / dout (backward), so it runs on a side stream next to the
-# memory-bound routing and gather kernels of the routed path and is joined before the combine.
+# memory-bound routing and gather kernels of the routed path and is joined before the combine.  The same stream takes
+# the router's gradient and, in a forward pass of few tokens, the experts of many rows.
 OVERLAP_SHARED = True
 _SIDE = {}
 
@@ -251,6 +252,9 @@ class LayerCache:
   aux_loss: torch.Tensor      # f32 [1], unweighted load-balance loss
 
   def item(self, name, dtype, shape):
+    if name == "xs":   # (a forward pass of few tokens does not write it)
+      tb = self.tables
+      return ops.dispatch_rows(self.x, tb.pad_pos.view(-1, self.k), tb.row_slot, n_rows_dev=tb.n_blocks, rows_per_unit=BLOCK).view(dtype).view(*shape)
     i = _RES_NAMES.index(name)
     n = 1
     for v in shape:
@@ -285,8 +289,8 @@ def _dims(x, w: MoEWeights, k):
   return int(t), int(d), int(e), int(f), int(k), int(fs)
 
 
-def _streams(device, shared):
-  side = _side_stream(device).cuda_stream if (OVERLAP_SHARED and shared) else None
+def _streams(device):
+  side = _side_stream(device).cuda_stream if OVERLAP_SHARED else None
   return stream(), side
 
 
@@ -307,7 +311,7 @@ def moe_layer_fwd(x, w: MoEWeights, k, prepared=True):
   out = torch.empty_like(x)
   aux = torch.empty(1, dtype=torch.float32, device=dev)
   prep = _prepared_router(w.w_router) if prepared else None
-  main, side = _streams(dev, fs > 0)
+  main, side = _streams(dev)
   check(lib.lewi_moe_fwd(main, side, ptr(x), ptr(w.w_router), ptr(w.router_bias), ptr(prep), ptr(w.w_gate), ptr(w.w_up),
                          ptr(w.w_down), ptr(w.ws_gate), ptr(w.ws_up), ptr(w.ws_down), ptr(w.w_sg), ptr(out), ptr(aux),
                          ptr(residual), residual.numel(), ptr(ws), ws.numel(), *dims), "lewi_moe_fwd")
@@ -334,7 +338,7 @@ def moe_layer_bwd(dout, w: MoEWeights, c: LayerCache, aux_grad=0.0, wgrad_dtype=
     g["drouter_bias"] = torch.empty(e, dtype=torch.float32, device=dev)
   ws = _workspace(int(lib.lewi_moe_workspace_bytes(*dims, int(w.w_sg is not None))), dev)
   prep = _prepared_router(w.w_router) if prepared else None
-  main, side = _streams(dev, fs > 0)
+  main, side = _streams(dev)
   check(lib.lewi_moe_bwd(main, side, ptr(dout), ptr(c.x), ptr(w.w_router), ptr(prep), ptr(w.w_gate), ptr(w.w_up),
                          ptr(w.w_down), ptr(w.ws_gate), ptr(w.ws_up), ptr(w.ws_down), ptr(w.w_sg), ptr(c.residual),
                          c.residual.numel(), ptr(ws), ws.numel(), ptr(g["dx"]), ptr(g["dw_router"]),

@@ -1,0 +1,66 @@
+"""Forward passes of few tokens: the kernels that stream weights past a block's rows (few_gemm.cuh), against the oracle and
+against the pair kernels.  Sizes sit where a rule or a tile ends: one row, 16 and 17 rows, a block and a row more, the
+last token count that takes every expert (512) and the first that leaves those of several blocks to the pair kernels,
+contractions and widths that fill no tile."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+from test_gpu_layer import compare, run_layer
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("t,d,e,f,fs,k,skew", [
+    (1, 64, 64, 64, 64, 2, False), (17, 136, 8, 72, 40, 2, False), (16, 192, 64, 200, 64, 3, False), (128, 256, 64, 128, 192, 2, True),
+    (129, 256, 16, 72, 64, 4, True), (512, 128, 64, 64, 64, 2, True), (513, 128, 64, 64, 64, 2, True), (700, 256, 64, 136, 72, 4, True)])
+def test_layer_of_few_tokens_against_the_oracle(cuda, t, d, e, f, fs, k, skew):
+  bias = O.zipf_bias(e, seed=0) if skew else None
+  inp, out, cache, grads, want, c, g = run_layer(cuda, t, d, e, f, fs, k, seed=t, bias=bias, router_scale=5.0)
+  compare(out, cache, grads, want, c, g, k)
+  if t > 512:   # both kinds of experts
+    assert c["gs"].max() > 128 and ((c["gs"] > 0) & (c["gs"] <= 128)).any()
+
+
+@pytest.mark.parametrize("t,d,e,f,k,skew,side", [(1, 1024, 128, 512, 6, False, True), (33, 264, 16, 136, 6, False, True),
+                                                 (130, 1024, 64, 512, 6, True, True), (512, 256, 32, 128, 6, True, True),
+                                                 (600, 1024, 64, 512, 6, True, True), (600, 1024, 64, 512, 6, True, False),
+                                                 (1300, 512, 128, 256, 6, False, True)])
+def test_few_rows_give_the_pair_kernels_bits(cuda, monkeypatch, t, d, e, f, k, skew, side):
+  """Sums run over the same 16-deep steps in the same order: g|u, h and the output are equal, not close; rows of h without a slot are zero.
+  (Residuals of a fresh allocation: what earlier calls left there must not show.)"""
+  from lewi_surge_b200 import layer, ops
+  monkeypatch.setattr(layer, "OVERLAP_SHARED", side)
+  gen = torch.Generator(device=cuda).manual_seed(t)
+  rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda).bfloat16()
+  bias = torch.from_numpy(O.zipf_bias(e, seed=0)).float().to(cuda) if skew else None
+  w = layer.MoEWeights(rnd(d, e).float() * 0.02, rnd(e, d, f) * 0.02, rnd(e, d, f) * 0.02, rnd(e, f, d) * 0.02, router_bias=bias)
+  x = rnd(t, d)
+  junk = torch.full((64 << 20,), float("nan"), device=cuda, dtype=torch.float32)
+  del junk
+  out, cache = layer.moe_layer_fwd(x, w, k)
+  tb = cache.tables
+  xs = ops.dispatch_rows(x, tb.pad_pos.view(t, k), tb.row_slot)
+  live = int(tb.n_blocks.item()) * 128
+  gu, h = layer.gateup_swiglu(xs, w.w_gate, w.w_up, tb.block_expert, tb.n_blocks, pad_offsets=tb.pad_offsets, h_scale_src=tb.topk_w,
+                              scale_idx=tb.row_slot)
+  ys = ops.grouped_gemm_nn(h, w.w_down, tb.block_expert, tb.n_blocks, pad_offsets=tb.pad_offsets)
+  want = ops.gather_reduce(ys, tb.pad_pos.view(t, k))
+  rows = torch.nonzero(tb.row_slot[:live] >= 0).flatten()
+  assert torch.equal(cache.item("gu", torch.bfloat16, (tb.mpad, 2 * f))[rows], gu[rows])
+  assert torch.equal(cache.item("h", torch.bfloat16, (tb.mpad, f))[:live], h[:live])
+  assert torch.equal(cache.item("xs", torch.bfloat16, (tb.mpad, d))[:live], xs[:live])
+  assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("t,d,e", [(1, 64, 64), (16, 128, 128), (17, 192, 64), (130, 1024, 512), (3000, 320, 128)])
+def test_router_logits_of_few_tokens(cuda, t, d, e):
+  """1e-5 of a float64 product, with a bias; 192 and 320 are an odd number of 64-deep steps."""
+  from lewi_surge_b200 import layer
+  gen = torch.Generator(device=cuda).manual_seed(t)
+  x = torch.randn(t, d, generator=gen, device=cuda).bfloat16()
+  w, b = torch.randn(d, e, generator=gen, device=cuda), torch.randn(e, generator=gen, device=cuda)
+  want = x.double() @ w.double() + b.double()
+  got = layer.router_logits(x, w, b)
+  assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
