@@ -77,6 +77,19 @@ inline int num_sms() {
   return cached[dev];
 }
 
+// raises the dynamic shared memory limit of a kernel once per device
+template <class Kern>
+inline bool allow_smem(Kern kern, int bytes, bool (&done)[64]) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (done[dev]) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return done[dev] = true;
+}
+
 // Host-side count of kernel launches made through this library (read by lewi_launch_count()).
 inline long long& launch_counter() {
   static long long n = 0;
