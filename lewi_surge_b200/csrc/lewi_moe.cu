@@ -771,10 +771,7 @@ int lewi_grouped_gemm_tn(void* stream, const void* a_ptr, const void* b_ptr, voi
     gg::tn_reduce_kernel<<<(int)grid, 256, 0, st>>>(a.partial, splits, (long long)E * Ma, Nb, out, out2, a.out_f32);
     LEWI_CHECK_LAUNCH();
   } else if (part_rows > 0) {
-    long long gx = ((long long)Ma * Nb / 4 + 255) / 256;
-    if (gx > 32) gx = 32;
-    gg::tn_reduce_ragged_kernel<<<dim3((unsigned)gx, (unsigned)E), 256, 0, st>>>(a.partial, pad_offsets, E, part_rows, Ma, Nb,
-                                                                                 out, out2, a.out_f32);
+    gg::tn_reduce_ragged_kernel<<<4 * num_sms(), 256, 0, st>>>(a.partial, pad_offsets, E, part_rows, Ma, Nb, out, out2, a.out_f32);
     LEWI_CHECK_LAUNCH();
   }
   return LEWI_OK;
