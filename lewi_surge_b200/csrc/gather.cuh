@@ -89,20 +89,21 @@ __global__ void __launch_bounds__(kGatherThreads) gather_rows_kernel(
 // (row_slot[r] < 0) become zero rows.  Every output row has exactly one writer, so this is the same function as
 // the row gather out[r] = x[row_slot[r] / k] -- but each source row is read once instead of k times at k distant
 // moments, which keeps the read side at T rows of DRAM traffic however large the source is against the L2.
-// A warp looks at ZR rows at a time for those to zero: 4 while no warp of the grid looks more than twice (kZeroRows), since at decode
+// (5003 tokens, k = 6, d = 1024, float32, no padding: 23 us, the row gather 35; 16,384 tokens, k = 12, d = 2048, bf16: 140 and 240.)
+// row_slot null: there are none.  A warp looks at ZR rows at a time for those to zero: 4 while no warp of the grid looks more than twice (kZeroRows), since at decode
 // sizes nearly all rows are such rows (8 tokens over 128 experts: 6.1 MB of zeros; 13 us with 32 rows per warp, 7 us with 4);
 // 32 beyond, where hardly any are (k = 6, d = 256: 16,384 tokens over 16 experts 9.3 us with 4 and 9.8 with 32, 49,152 34 and 32,
 // 65,536 over 128 48 and 45).
 constexpr int kZeroRows = 4;
-template <int VPL, int ZR>
+template <typename T, int VPL, int ZR>
 __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
-    const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
-    __nv_bfloat16* __restrict__ out, long long n_tokens, int k, int d, long long out_rows,
+    const T* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
+    T* __restrict__ out, long long n_tokens, int k, int d, long long out_rows,
     const int32_t* __restrict__ n_rows_dev, int rows_per_unit) {
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int nvec = d / 8;
+  const int nvec = d / Elem<T>::kPerVec;
   long long rows = out_rows;
   if (n_rows_dev != nullptr) rows = min(rows, (long long)n_rows_dev[0] * rows_per_unit);
   for (long long t = warp0; t < n_tokens; t += n_warps) {
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
       }
     }
   }
+  if (row_slot == nullptr) return;
   // zero rows of the padded layout
   for (long long r0 = warp0 * ZR; r0 < rows; r0 += n_warps * ZR) {
     const long long r = r0 + lane;
@@ -356,6 +358,78 @@ inline int gather_grid(long long rows) {
 }
 
 // smallest supported VPL in {1,2,4,8,16} covering the row, or 0
+// Gradients of the combine, both in one pass over y, in token order: dy[pos[t,j]] = w[t,j] * g[t] and dw[t,j] = <g[t], y[pos[t,j]]>,
+// g in y's type (a float32 g is rounded here).  pos is a permutation, so every row of dy has one writer; a row of g is read once, not
+// k times, and a warp requests the next row of y while it works on one.
+// 5003 tokens, k = 6, d = 1024, float32: 47 us (scaled gather and dots 35 + 39); 16,384 tokens, k = 12, d = 2048, bf16: 328 us, 5.3 TB/s
+// (240 + 207 and 32 for the rounded copy of g).  A warp per row of y instead, g out of L2 k times: 55 and 472 us.
+template <typename T, typename TG, int VPL>
+__global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __restrict__ y, const int32_t* __restrict__ pos,
+                                                                     const TG* __restrict__ g, const float* __restrict__ w,
+                                                                     T* __restrict__ dy, float* __restrict__ dw, long long n, int k, int d) {
+  constexpr int PV = Elem<T>::kPerVec, GV = PV * sizeof(TG) / 16;   // vectors of g per vector of y
+  const int lane = threadIdx.x & 31;
+  const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5, m = n * k;
+  const int nvec = d / PV;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (long long t = warp0; t < n; t += n_warps) {
+    const int my_pos = lane < k ? pos[t * k + lane] : -1;
+    const float my_w = lane < k ? w[t * k + lane] : 0.f;
+    uint4 gv[VPL], yv[VPL], next[VPL];
+    auto fetch = [&](int j, uint4 (&v)[VPL]) {
+      const long long p = __shfl_sync(0xffffffffu, my_pos, j);
+#pragma unroll
+      for (int c = 0; c < VPL; ++c) {
+        const int vi = lane + c * kWarp;
+        v[c] = vi < nvec && p >= 0 && p < m ? ld_nc_v4(reinterpret_cast<const uint4*>(y + p * d) + vi) : zero;
+      }
+    };
+    fetch(0, yv);
+#pragma unroll
+    for (int c = 0; c < VPL; ++c) {
+      const int vi = lane + c * kWarp;
+      if (vi >= nvec) gv[c] = zero;
+      else if constexpr (GV == 2) {   // float32 -> bf16
+        const uint4* src = reinterpret_cast<const uint4*>(g + t * d) + (long long)vi * 2;
+        const uint4 a = ld_nc_v4(src), b = ld_nc_v4(src + 1);
+        auto two = [](uint32_t lo, uint32_t hi) { return pack_bf16(__uint_as_float(lo), __uint_as_float(hi)); };
+        gv[c] = make_uint4(two(a.x, a.y), two(a.z, a.w), two(b.x, b.y), two(b.z, b.w));
+      } else {
+        gv[c] = ld_nc_v4(reinterpret_cast<const uint4*>(g + t * d) + vi);
+      }
+    }
+    float my_dot = 0.f;
+    for (int j = 0; j < k; ++j) {
+      if (j + 1 < k) fetch(j + 1, next);
+      const long long p = __shfl_sync(0xffffffffu, my_pos, j);
+      const float s = __shfl_sync(0xffffffffu, my_w, j);
+      const bool in = p >= 0 && p < m;
+      if (p >= m && lane == 0) raise_status(LEWI_STATUS_BAD_INDEX);
+      float dot = 0.f;
+#pragma unroll
+      for (int c = 0; c < VPL; ++c) {
+        const int vi = lane + c * kWarp;
+        if (vi < nvec && in) {
+          float f[PV], q[PV];
+          Elem<T>::unpack(yv[c], f);
+          Elem<T>::unpack(gv[c], q);
+#pragma unroll
+          for (int e = 0; e < PV; ++e) {
+            dot = fmaf(q[e], f[e], dot);
+            q[e] *= s;
+          }
+          st_v4(reinterpret_cast<uint4*>(dy + p * d) + vi, Elem<T>::pack(q));
+        }
+        yv[c] = next[c];
+      }
+      dot = warp_sum(dot);
+      if (lane == j) my_dot = dot;
+    }
+    if (lane < k) dw[t * k + lane] = my_dot;
+  }
+}
+
 // Padded rows of the experts that have more than one row block: row r = x[row_slot[r] / k], zeros where row_slot[r] < 0; other experts'
 // blocks are passed over.  A CTA takes 16 rows, two per warp (a block per CTA, 16 rows per warp: 15 us instead of 4 for eight experts of
 // 700 rows, and the experts' GEMMs wait for it).

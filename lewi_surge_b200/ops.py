@@ -132,6 +132,32 @@ def gather_dot(y, pos, g):
   return out
 
 
+def dispatch_tokens(x, pos, k):
+  """out[pos[t*k+j]] = x[t] for a permutation pos of the N*k rows: equals ``gather_rows(x, order, idx_div=k)`` for its inverse, reading
+  every row once."""
+  lib = _lib.load()
+  x, pos = x.contiguous(), _i32(pos).contiguous()
+  t, d = x.shape
+  out = torch.empty((t * k, d), dtype=x.dtype, device=x.device)
+  check(lib.lewi_dispatch_tokens(stream(), ptr(x), ptr(pos), ptr(out), t, k, d, _dt(x)), "lewi_dispatch_tokens")
+  return out
+
+
+def combine_bwd(y, pos, g, w):
+  """(dy, dw f32) of ``combine`` for a permutation pos (N, k): dy[pos[t,j]] = w[t,j] * g[t], dw[t,j] = <g[t], y[pos[t,j]]>, g rounded to
+  y.dtype."""
+  lib = _lib.load()
+  y, pos, w = y.contiguous(), _i32(pos).contiguous(), w.to(torch.float32).contiguous()
+  g = (g if g.dtype in (y.dtype, torch.float32) else g.to(y.dtype)).contiguous()
+  (n, k), d = w.shape, y.shape[1]
+  if y.shape[0] != n * k or pos.numel() != n * k or g.shape != (n, d):
+    raise LewiError("combine_bwd: y (N*k, D), pos (N, k), g (N, D), w (N, k)")
+  dy, dw = torch.empty_like(y), torch.empty_like(w)
+  if n * k > 0:
+    check(lib.lewi_combine_bwd(stream(), ptr(y), ptr(pos), ptr(g), ptr(w), ptr(dy), ptr(dw), n, k, d, _dt(y), _dt(g)), "lewi_combine_bwd")
+  return dy, dw
+
+
 def sort_indices(flat_experts, num_experts=None, method=None):
   """Stable sort of the N*k expert slots by expert id -> (order, pos).
 
@@ -167,6 +193,8 @@ class _Dispatch(torch.autograd.Function):
     k = order.shape[0] // n
     ctx.save_for_backward(pos)
     ctx.n, ctx.k, ctx.dtype = n, k, x.dtype
+    if 0 < k <= 32 and k * n == order.shape[0] == pos.shape[0]:
+      return dispatch_tokens(x, pos, k)
     return gather_rows(x, order, idx_div=k)
 
   @staticmethod
@@ -176,23 +204,19 @@ class _Dispatch(torch.autograd.Function):
 
 
 class _Combine(torch.autograd.Function):
-  """y: (N*k, D) sorted rows, w: (N, k) -> (N, D) f32.  Backward: scaled gather (dy) and gather_dot (dw)."""
+  """y: (N*k, D) sorted rows, w: (N, k) -> (N, D) f32.  Backward: scaled gather (dy) and dots (dw) in one pass over y."""
 
   @staticmethod
   def forward(ctx, y, order, pos, w):
     n, k = w.shape
-    ctx.save_for_backward(y, order, pos, w)
+    ctx.save_for_backward(y, pos, w)
     return gather_reduce(y, pos.view(n, k), w, torch.float32)
 
   @staticmethod
   def backward(ctx, g):
-    y, order, pos, w = ctx.saved_tensors
-    n, k = w.shape
-    gy = g.to(y.dtype).contiguous()
-    # dy[p] = w_flat[order[p]] * g[order[p] // k]
-    dy = gather_rows(gy, order, w.reshape(-1), idx_div=k, scale_by_idx=True)
-    dw = gather_dot(y, pos.view(n, k), gy).to(w.dtype)
-    return dy, None, None, dw
+    y, pos, w = ctx.saved_tensors
+    dy, dw = combine_bwd(y, pos, g, w)
+    return dy, None, None, dw.to(w.dtype)
 
 
 class _PermuteRows(torch.autograd.Function):

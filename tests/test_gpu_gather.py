@@ -156,3 +156,29 @@ def test_gather_reduce_of_few_rows_gives_the_bits_of_many(cuda, dtype, out, k):
   for r in (1, 3, 700):
     assert torch.equal(ops.gather_reduce(y, pos[:r], w[:r], out, add0=a0[:r], add1=a1[:r]), many[:r])
     assert torch.equal(ops.gather_reduce(y, pos[:r], None, out), bare[:r])
+
+
+@pytest.mark.parametrize("t,k,d,dtype,g_dtype", [(1, 1, 8, "bf16", "f32"), (3, 32, 4, "f32", "f32"), (33, 7, 264, "bf16", "bf16"),
+                                                 (700, 6, 1032, "bf16", "f32"), (129, 12, 1028, "f32", "f32"), (70, 6, 2048, "f32", "f32"), (60, 6, 4096, "bf16", "f32"),
+                                                 (2500, 3, 256, "f32", "f32")])
+def test_token_order_dispatch_and_combine_gradients_equal_the_row_gathers(cuda, t, k, d, dtype, g_dtype):
+  """Same bits as gather_rows / scaled gather_rows / gather_dot on the inverse permutation, through the public functions' gradients too."""
+  from lewi_surge_b200 import ops, _lib
+  dt = dict(bf16=torch.bfloat16, f32=torch.float32)
+  gen = torch.Generator(device=cuda).manual_seed(t + k)
+  order = torch.randperm(t * k, generator=gen, device=cuda).to(torch.int32)
+  pos = torch.empty_like(order)
+  pos[order.long()] = torch.arange(t * k, dtype=torch.int32, device=cuda)
+  rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda)
+  x, y, w, g = rnd(t, d).to(dt[dtype]), rnd(t * k, d).to(dt[dtype]), rnd(t, k), rnd(t, d).to(dt[g_dtype])
+  _lib.last_status()
+  assert torch.equal(ops.dispatch(x, order, pos), ops.gather_rows(x, order, idx_div=k))
+  gy = g.to(y.dtype)
+  dy, dw = ops.combine_bwd(y, pos.view(t, k), g, w)
+  assert torch.equal(dy, ops.gather_rows(gy, order, w.reshape(-1), idx_div=k, scale_by_idx=True))
+  assert torch.equal(dw, ops.gather_dot(y, pos.view(t, k), gy))
+  y.requires_grad_(True)
+  w.requires_grad_(True)
+  got = torch.autograd.grad(ops.combine(y, order, pos, w), (y, w), g.float())
+  assert torch.equal(got[0], dy) and torch.equal(got[1], dw)
+  assert _lib.last_status() == 0
