@@ -310,13 +310,13 @@ bwd_scans_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 // ------------------------------------------------------------------------------------------------ chunk kernel
 
 constexpr int kBwdThreads = 512;
-constexpr int kHalfBox = 32 * 128;   // a [32 rows][64 bf16] tile
+constexpr int kVBox = 16 * 128;      // a [16 rows][64 bf16] tile
 
 // Shared memory: tiles k, q*scale, k*beta, v*beta, do; the pieces of A; the pieces of dvb (later those of T and dP); the stage
-// (32 columns of V at a time: pieces of h_in, dh, v_new; before that S, A and scratch in float32; later the pieces of dkg, then
+// (two buffers for 16 columns of V each: pieces of h_in, dh, v_new; before that S, A and scratch in float32; later the pieces of dkg, then
 // those of X); gates, beta and the partial sums.
 struct BwdSmem {
-  int k, q, kb, vb, d_o, a, dvb, t, dp, stage, sh, sdh, svn, gates, beta, red, total;
+  int k, q, kb, vb, d_o, a, dvb, t, dp, stage, sh, sdh, svn, vbuf, gates, beta, red, total;
 };
 __host__ __device__ constexpr BwdSmem bwd_smem(int kboxes, int vboxes) {
   BwdSmem m{};
@@ -330,10 +330,11 @@ __host__ __device__ constexpr BwdSmem bwd_smem(int kboxes, int vboxes) {
   m.t = m.dvb;
   m.dp = m.dvb + 3 * kBox;
   m.stage = m.dvb + 6 * kBox;
-  m.sh = m.stage;
-  m.sdh = m.sh + 3 * kboxes * kHalfBox;
-  m.svn = m.sdh + 3 * kboxes * kHalfBox;
-  const int stage_end = m.svn + 3 * kHalfBox, scratch_end = m.stage + (2 * C + 32) * kSP * 4;
+  m.sh = 0;   // within one of the two buffers of the stage
+  m.sdh = m.sh + 3 * kboxes * kVBox;
+  m.svn = m.sdh + 3 * kboxes * kVBox;
+  m.vbuf = m.svn + 3 * kVBox;
+  const int stage_end = m.stage + 2 * m.vbuf, scratch_end = m.stage + (2 * C + 32) * kSP * 4;
   m.gates = stage_end > scratch_end ? stage_end : scratch_end;
   m.beta = m.gates + kGateBytes;
   m.red = m.beta + C * 4;
@@ -380,11 +381,13 @@ __device__ __forceinline__ float quad_sum(float v) {
 
 // One CTA of 16 warps per chunk and head.  [64, K] results: warp (wm, wc) owns 16 tokens and a quarter of the columns;
 // [64, 64] results: one 16 x 16 tile.  What contracts over V (dqE, dkg, dkd, dattn: 8,000 of the 12,600 MMAs at K = V = 128)
-// runs over 32 columns at a time, whose pieces of h_in, dh and v_new all warps cut and share.
+// runs over 16 columns at a time, whose pieces of h_in, dh and v_new all warps cut and share.
 // dqE, dkg and dkd are summed up by the tensor core: they leave in bf16, and dg, which takes their row sums, is no further from 64 bits
 // for it (2.3e-7 of its norm at 512 tokens, K = V = 128; 3.8e-7 in float32 on the CUDA cores; summed up with rounding 1.9e-7, and
 // this kernel 1.10 ms).  The [64, 64] sums, whose results are cut into pieces again, are rounded (gdn_mma.cuh).
-// B=8, S=4096, H=8, K=V=128: 1.03 ms (4.43 ms in float32 on the CUDA cores).
+// B=8, S=4096, H=8, K=V=128: 0.96 ms (4.43 ms in float32 on the CUDA cores; 1.04 with 32 columns of V between two barriers that all
+// cut and then all multiplied, tiles of the [64, 64] matrices by quarters, and loads where they are used).  Of 63,500 cycles a chunk the
+// loop over V takes 25,500 for 16,300 of MMAs, dvb 6,600, X 5,500.
 template <int KB, int VB, bool ANY>
 __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs g) {
   extern __shared__ __align__(1024) uint8_t gdn_smem_raw[];
@@ -412,7 +415,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   const int n = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp & 3, wc = warp >> 2;
-  const bool active = wc <= wm;                       // this warp's 16 x 16 tile is not above the diagonal
+  // this warp's 16 x 16 tile of the [64, 64] matrices: the ten that are not above the diagonal come first, which spreads them over the
+  // schedulers (3, 3, 2 and 2; by quarters it would be 1, 2, 3 and 4)
+  const int tm = (int)(0x940ffa94u >> (2 * warp) & 3), tc = (int)(0xfb9e4910u >> (2 * warp) & 3);
+  const bool active = tc <= tm;
   const int er = lane >> 2, ec = (lane & 3) * 2;      // this lane's elements of an accumulator tile
   const LaneOff L = lane_off(lane);
   const Dims& D = g.D;
@@ -467,6 +473,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   }
   __syncthreads();
 
+  // dv_new of this warp's 16 columns of V (see below), requested long before it is used
+  const int nvb = (BW.v16 + 1) / 2, dblk = warp >> 1;   // blocks of 32 columns of V; the warp's block of 16
+  float4 dvt[8];
+  {
+    const float4* src = reinterpret_cast<const float4*>(g.bws + BW.dv) + (chunk * BW.v16 + dblk) * 8 * 32 + lane;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) dvt[t] = dblk < BW.v16 ? src[t * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+
   // ---- bf16(kb k^T) and P = bf16(q k^T), kept as packed bf16; S to shared memory
   uint32_t ps[4] = {0, 0, 0, 0}, pa[4] = {0, 0, 0, 0};
   auto decay = [&](int r, int c) { return __expf(gcs[r] - gcs[c]); };
@@ -475,9 +490,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
     zero4(s2[0]); zero4(s2[1]); zero4(a2[0]); zero4(a2[1]);
 #pragma unroll
     for (int ks = 0; ks < 4 * KB; ++ks) {
-      const Frag4 bb = ld_b(tK, wc * 16, ks, L);
-      mma2_add(s2[0], s2[1], ld_a(tKb, wm * 16, ks, L).r, bb);
-      mma2_add(a2[0], a2[1], ld_a(tQ, wm * 16, ks, L).r, bb);
+      const Frag4 bb = ld_b(tK, tc * 16, ks, L);
+      mma2_add(s2[0], s2[1], ld_a(tKb, tm * 16, ks, L).r, bb);
+      mma2_add(a2[0], a2[1], ld_a(tQ, tm * 16, ks, L).r, bb);
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -485,7 +500,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
       for (int e = 0; e < 2; ++e) {
         ps[t * 2 + e] = pack_bf16(s2[t][2 * e], s2[t][2 * e + 1]);
         pa[t * 2 + e] = pack_bf16(a2[t][2 * e], a2[t][2 * e + 1]);
-        const int r = wm * 16 + er + 8 * e, c = wc * 16 + t * 8 + ec;
+        const int r = tm * 16 + er + 8 * e, c = tc * 16 + t * 8 + ec;
         *reinterpret_cast<float2*>(sS + r * kSP + c) =
             make_float2(c < r ? bf16_lo(ps[t * 2 + e]) * decay(r, c) : 0.f, c + 1 < r ? bf16_hi(ps[t * 2 + e]) * decay(r, c + 1) : 0.f);
       }
@@ -505,19 +520,37 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   __syncthreads();
 
   // ---- dvb = A^T dv_new: warp = (16 columns of V, 32 of the tokens); its pieces to shared memory, dv, part of dbeta
-  const int nvb = (BW.v16 + 1) / 2;                   // blocks of 32 columns of V
+  // what the first pass over V needs is requested here
+  const float4* hs_in = reinterpret_cast<const float4*>(g.bws + BW.hs) + chunk * BW.v16 * (8 * KB) * 32 + warp * 32 + lane;
+  const float4* dh_in = reinterpret_cast<const float4*>(g.bws + BW.dh) + chunk * BW.v16 * (8 * KB) * 32 + warp * 32 + lane;
+  const float4* vn_in = reinterpret_cast<const float4*>(g.bws + BW.vn) + chunk * BW.v16 * 8 * 32 + warp * 32 + lane;
+  float4 hr, dr, vr;   // this warp's tile of h_in^T, dh^T and (the first eight warps) v_new^T
+  auto fetch = [&](int vb) {
+    if (warp < 8 * KB) {
+      hr = hs_in[vb * (8 * KB) * 32];
+      dr = dh_in[vb * (8 * KB) * 32];
+    }
+    if (warp < 8) vr = vn_in[vb * 8 * 32];
+  };
+  fetch(0);
   {
-    const int blk = warp >> 1;
+    const int blk = dblk;
     if (blk < 2 * nvb) {
-      const float4* src = reinterpret_cast<const float4*>(g.bws + BW.dv) + (chunk * BW.v16 + blk) * 8 * 32 + lane;
-      float4 dvt[8];
+      // token blocks 0, 3 or 1, 2 (A^T is upper triangular: the sum of block m runs over m..3)
+      const int mrow[2] = {warp & 1, 3 - (warp & 1)};
+      uint32_t vv[2][2][2];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) dvt[t] = blk < BW.v16 ? src[t * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const int r = mrow[x] * 16 + er + 8 * e, c = blk * 16 + t * 8 + ec;
+            vv[x][e][t] = in_seq(r) && c < V ? *reinterpret_cast<const uint32_t*>(g.v + row_off(r) * V + c) : 0u;
+          }
       float acc[2][2][4];
 #pragma unroll
       for (int x = 0; x < 2; ++x) { zero4(acc[x][0]); zero4(acc[x][1]); }
-      // token blocks 0, 3 or 1, 2 (A^T is upper triangular: the sum of block m runs over m..3)
-      const int mrow[2] = {warp & 1, 3 - (warp & 1)};
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint32_t b0[3][2], b1[3][2];   // an accumulator tile of dv^T is the B operand of this product
@@ -546,9 +579,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
             const float d0 = acc[x][t][2 * e], d1 = acc[x][t][2 * e + 1];
             put_pieces(tDvb + (c >> 6) * kBox, VB * kBox, r, c & 63, d0, d1);
             if (in_seq(r) && c < V) {
-              const uint32_t vv = *reinterpret_cast<const uint32_t*>(g.v + row_off(r) * V + c);
-              rb = fmaf(d0, bf16_lo(vv), rb);
-              rb = fmaf(d1, bf16_hi(vv), rb);
+              rb = fmaf(d0, bf16_lo(vv[x][e][t]), rb);
+              rb = fmaf(d1, bf16_hi(vv[x][e][t]), rb);
               st_pair<ANY>(g.dv + row_off(r) * V + c, pack_bf16(d0 * be, d1 * be));
             }
           }
@@ -558,84 +590,66 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
     }
   }
 
-  // ---- over V, 32 columns at a time: dqE = do h_in^T, -dkg = dvb h_in^T, dkd = v_new dh^T, dattn = do v_new^T
+  // ---- over V, 16 columns at a time: dqE = do h_in^T, -dkg = dvb h_in^T, dkd = v_new dh^T, dattn = do v_new^T.  Two buffers: while a
+  // block is multiplied the pieces of the next one are cut into the other, and the one after that is on its way from memory.
   float dq[2 * KB][4], dkb[2 * KB][4], dk[2 * KB][4], dat[2][4];
 #pragma unroll
   for (int t = 0; t < 2 * KB; ++t) { zero4(dq[t]); zero4(dkb[t]); zero4(dk[t]); }
   zero4(dat[0]); zero4(dat[1]);
   float hd = 0.f;                                     // <dh, h_in>
   {
-    const float4* hs_in = reinterpret_cast<const float4*>(g.bws + BW.hs) + chunk * BW.v16 * (8 * KB) * 32;
-    const float4* dh_in = reinterpret_cast<const float4*>(g.bws + BW.dh) + chunk * BW.v16 * (8 * KB) * 32;
-    const float4* vn_in = reinterpret_cast<const float4*>(g.bws + BW.vn) + chunk * BW.v16 * 8 * 32;
-    // thread's tiles of a block: state tile (warp + 16*x) of 2 x 8*KB, v_new tile (warp) of 2 x 8
-    float4 hr[KB], dr[KB], vr;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto fetch = [&](int vb) {
-#pragma unroll
-      for (int x = 0; x < KB; ++x) {
-        const int t = warp + 16 * x;                  // (16-column block, tile) of the pair of blocks
-        const bool in = 2 * vb + t / (8 * KB) < BW.v16;
-        const long long at = ((long long)2 * vb * (8 * KB) + t) * 32 + lane;
-        hr[x] = in ? hs_in[at] : zero;
-        dr[x] = in ? dh_in[at] : zero;
+    auto put = [&](int vb) {
+      const uint32_t buf = tStage + (vb & 1) * M.vbuf;
+      const int c = (warp & 7) * 8 + ec;
+      if (warp < 8 * KB) {
+        const uint32_t box = (warp >> 3) * kVBox;
+        put_pieces(buf + M.sh + box, KB * kVBox, er, c, hr.x, hr.y);
+        put_pieces(buf + M.sh + box, KB * kVBox, er + 8, c, hr.z, hr.w);
+        put_pieces(buf + M.sdh + box, KB * kVBox, er, c, dr.x, dr.y);
+        put_pieces(buf + M.sdh + box, KB * kVBox, er + 8, c, dr.z, dr.w);
+        hd = fmaf(hr.x, dr.x, hd); hd = fmaf(hr.y, dr.y, hd);
+        hd = fmaf(hr.z, dr.z, hd); hd = fmaf(hr.w, dr.w, hd);
       }
-      vr = 2 * vb + warp / 8 < BW.v16 ? vn_in[((long long)2 * vb * 8 + warp) * 32 + lane] : zero;
+      if (warp < 8) {
+        put_pieces(buf + M.svn, kVBox, er, c, vr.x, vr.y);
+        put_pieces(buf + M.svn, kVBox, er + 8, c, vr.z, vr.w);
+      }
     };
-    fetch(0);
-    for (int vb = 0; vb < nvb; ++vb) {
-      __syncthreads();   // the stage is free (first: the float32 scratch is dead, the pieces of dvb are complete)
+    __syncthreads();   // the float32 scratch is dead
+    put(0);
+    if (BW.v16 > 1) fetch(1);
+    __syncthreads();   // (the pieces of dvb are complete, too)
+    for (int ks = 0; ks < BW.v16; ++ks) {
+      const uint32_t buf = tStage + (ks & 1) * M.vbuf;
+      if (ks + 1 < BW.v16) put(ks + 1);
+      if (ks + 2 < BW.v16) fetch(ks + 2);
+      const Frag4 fdo = ld_a(tDo, wm * 16, ks, L);
+      const Frag3x4 fdvb = ld_a3(tDvb, VB * kBox, wm * 16, ks, L), fvn = ld_a3_t(buf + M.svn, kVBox, 0, wm, L);
 #pragma unroll
-      for (int x = 0; x < KB; ++x) {
-        const int t = warp + 16 * x, tile = t % (8 * KB), r = t / (8 * KB) * 16 + er;
-        const uint32_t box = (tile >> 3) * kHalfBox;
-        const int c = (tile & 7) * 8 + ec;
-        put_pieces(base + M.sh + box, KB * kHalfBox, r, c, hr[x].x, hr[x].y);
-        put_pieces(base + M.sh + box, KB * kHalfBox, r + 8, c, hr[x].z, hr[x].w);
-        put_pieces(base + M.sdh + box, KB * kHalfBox, r, c, dr[x].x, dr[x].y);
-        put_pieces(base + M.sdh + box, KB * kHalfBox, r + 8, c, dr[x].z, dr[x].w);
-        hd = fmaf(hr[x].x, dr[x].x, hd); hd = fmaf(hr[x].y, dr[x].y, hd);
-        hd = fmaf(hr[x].z, dr[x].z, hd); hd = fmaf(hr[x].w, dr[x].w, hd);
+      for (int cp = 0; cp < KB; ++cp) {
+        const int np = wc * KB + cp;
+        Frag4 hb[3];
+#pragma unroll
+        for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(buf + M.sh + w3 * KB * kVBox, 0, np, L, kVBox);
+        mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[2]);
+        mma2_x6_acc(dkb[2 * cp], dkb[2 * cp + 1], fdvb, hb);
+        mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[1]);
+        mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[0]);
+#pragma unroll
+        for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(buf + M.sdh + w3 * KB * kVBox, 0, np, L, kVBox);
+        mma2_x6_acc(dk[2 * cp], dk[2 * cp + 1], fvn, hb);
       }
-      {
-        const int r = warp / 8 * 16 + er, c = (warp & 7) * 8 + ec;
-        put_pieces(base + M.svn, kHalfBox, r, c, vr.x, vr.y);
-        put_pieces(base + M.svn, kHalfBox, r + 8, c, vr.z, vr.w);
+      if (active) {
+        const Frag4 b[3] = {ld_b_t(buf + M.svn, 0, tc, L), ld_b_t(buf + M.svn + kVBox, 0, tc, L), ld_b_t(buf + M.svn + 2 * kVBox, 0, tc, L)};
+        mma2_x3(dat[0], dat[1], ld_a(tDo, tm * 16, ks, L).r, b);
       }
       __syncthreads();
-      if (vb + 1 < nvb) fetch(vb + 1);
-#pragma unroll
-      for (int k2 = 0; k2 < 2; ++k2) {
-        const int ks = vb * 2 + k2;
-        const Frag4 fdo = ld_a(tDo, wm * 16, ks, L);
-        const Frag3x4 fdvb = ld_a3(tDvb, VB * kBox, wm * 16, ks, L), fvn = ld_a3_t(base + M.svn, kHalfBox, k2 * 16, wm, L);
-#pragma unroll
-        for (int cp = 0; cp < KB; ++cp) {
-          const int np = wc * KB + cp;
-          Frag4 hb[3];
-#pragma unroll
-          for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(base + M.sh + w3 * KB * kHalfBox, k2 * 16, np, L, kHalfBox);
-          mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[2]);
-          mma2_x6_acc(dkb[2 * cp], dkb[2 * cp + 1], fdvb, hb);
-          mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[1]);
-          mma2(dq[2 * cp], dq[2 * cp + 1], fdo.r, hb[0]);
-#pragma unroll
-          for (int w3 = 0; w3 < 3; ++w3) hb[w3] = ld_b_t(base + M.sdh + w3 * KB * kHalfBox, k2 * 16, np, L, kHalfBox);
-          mma2_x6_acc(dk[2 * cp], dk[2 * cp + 1], fvn, hb);
-        }
-        if (active) {
-          const Frag4 b[3] = {ld_b_t(base + M.svn, k2 * 16, wc, L), ld_b_t(base + M.svn + kHalfBox, k2 * 16, wc, L),
-                              ld_b_t(base + M.svn + 2 * kHalfBox, k2 * 16, wc, L)};
-          mma2_x3(dat[0], dat[1], fdo.r, b);
-        }
-      }
     }
   }
   hd = warp_sum(hd);
   if (lane == 0) sHd[warp] = hd;
 
-  // ---- row sums, the decays of the rows, the pieces of dkg
-  __syncthreads();   // everybody is done with the stage
+  // ---- row sums, the decays of the rows, the pieces of dkg (everybody is done with the stage)
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const int r = wm * 16 + er + 8 * e;
@@ -668,13 +682,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   zero4(x1[0]); zero4(x1[1]); zero4(x2[0]); zero4(x2[1]);
   if (active) {
     for (int ks = 0; ks < 2 * nvb; ++ks) {
-      const Frag4 bb = ld_b(tVb, wc * 16, ks, L);
-      mma2_x3(x1[0], x1[1], ld_a3(tDvb, VB * kBox, wm * 16, ks, L), bb);
+      const Frag4 bb = ld_b(tVb, tc * 16, ks, L);
+      mma2_x3(x1[0], x1[1], ld_a3(tDvb, VB * kBox, tm * 16, ks, L), bb);
     }
 #pragma unroll
     for (int ks = 0; ks < 4 * KB; ++ks) {
-      const Frag4 bb = ld_b(tKb, wc * 16, ks, L);
-      mma2_x3(x2[0], x2[1], ld_a3(tStage, KB * kBox, wm * 16, ks, L), bb);
+      const Frag4 bb = ld_b(tKb, tc * 16, ks, L);
+      mma2_x3(x2[0], x2[1], ld_a3(tStage, KB * kBox, tm * 16, ks, L), bb);
     }
   }
   __syncthreads();   // dvb and dkg have been read: their places take T and X
@@ -685,7 +699,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
     for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int r = wm * 16 + er + 8 * e, c = wc * 16 + t * 8 + ec;
+        const int r = tm * 16 + er + 8 * e, c = tc * 16 + t * 8 + ec;
         put_pieces(tStage, kBox, r, c, fmaf(x2[t][2 * e], sE[c], x1[t][2 * e]), fmaf(x2[t][2 * e + 1], sE[c + 1], x1[t][2 * e + 1]));
         const float t0 = c <= r ? dat[t][2 * e] * decay(r, c) : 0.f, t1 = c + 1 <= r ? dat[t][2 * e + 1] * decay(r, c + 1) : 0.f;
         put_pieces(tT, kBox, r, c, t0, t1);
@@ -701,15 +715,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
   if (active) {
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
-      if (ks > wc) break;
-      const Frag4 b[3] = {ld_b(tA, wc * 16, ks, L), ld_b(tA + kBox, wc * 16, ks, L), ld_b(tA + 2 * kBox, wc * 16, ks, L)};
-      mma2_x6(ds[0], ds[1], ld_a3(tStage, kBox, wm * 16, ks, L), b);
+      if (ks > tc) break;
+      const Frag4 b[3] = {ld_b(tA, tc * 16, ks, L), ld_b(tA + kBox, tc * 16, ks, L), ld_b(tA + 2 * kBox, tc * 16, ks, L)};
+      mma2_x6(ds[0], ds[1], ld_a3(tStage, kBox, tm * 16, ks, L), b);
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int r = wm * 16 + er + 8 * e, c = wc * 16 + t * 8 + ec;
+        const int r = tm * 16 + er + 8 * e, c = tc * 16 + t * 8 + ec;
         const float p0 = c < r ? -ds[t][2 * e] * decay(r, c) : 0.f, p1 = c + 1 < r ? -ds[t][2 * e + 1] * decay(r, c + 1) : 0.f;
         put_pieces(tDp, kBox, r, c, p0, p1);
         gg[t][2 * e] = fmaf(p0, bf16_lo(ps[t * 2 + e]), gg[t][2 * e]);      // dS S = dP bf16(kb k^T)
@@ -719,7 +733,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const float rs = quad_sum(gg[0][2 * e] + gg[0][2 * e + 1] + gg[1][2 * e] + gg[1][2 * e + 1]);
-    if ((lane & 3) == 0) rowG[wc * C + wm * 16 + er + 8 * e] = rs;
+    if ((lane & 3) == 0) rowG[tc * C + tm * 16 + er + 8 * e] = rs;
   }
 #pragma unroll
   for (int t = 0; t < 2; ++t)
@@ -728,7 +742,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_chunk_kernel(const BwdArgs
       float cs = gg[t][e] + gg[t][2 + e];
 #pragma unroll
       for (int o = 4; o < 32; o <<= 1) cs += __shfl_xor_sync(0xffffffffu, cs, o);
-      if (lane < 4) colG[wm * C + wc * 16 + t * 8 + ec + e] = cs;
+      if (lane < 4) colG[tm * C + tc * 16 + t * 8 + ec + e] = cs;
     }
 
   // ---- dq += T k, dk += T^T q (rounded to bf16 next: accumulated by the tensor core, like dkb and dk below)
