@@ -233,6 +233,15 @@ int lewi_grouped_gemm_nt(void* stream, const void* a, const void* b, void* out, 
                          const int32_t* block_expert, const int32_t* n_blocks,
                          const int32_t* pad_offsets, int64_t rows, int K, int N, int E, int out_dtype);
 
+/* `jax.lax.ragged_dot` (modal/padded_gmm.py:45) on rows as they come, sorted by group and without padding: out[r] = a[r] . b[e] for
+ * offsets[e] <= r < offsets[e+1], zeros for r >= offsets[E]; a bf16 [m,K], out bf16 [m,N], b bf16 [E,K,N], or [E,N,K] with transposed.
+ * offsets i32 [E+1] on the device, as lewi_group_offsets writes them.  lewi_ragged_gemm_ok: 1 where it can be used (CTA pairs not
+ * switched off, sizes within their tables); otherwise pad the rows (lewi_group_tables). */
+int lewi_ragged_gemm_ok(int64_t m, int E);
+int lewi_group_offsets(void* stream, const int32_t* group_sizes, int E, int32_t* offsets);
+int lewi_ragged_gemm(void* stream, const void* a, const void* b, void* out, const int32_t* offsets, int64_t m, int K, int N, int E,
+                     int transposed);
+
 /* out[e] = a[rows of e]^T . b[rows of e]   a [rows,Ma], b [rows,Nb], out [E,Ma,Nb] (out_dtype).
  * pad_offsets i32 [E+1] gives each expert's padded row range (null: one group of all rows).
  * Experts without rows get zeros.  If out2 is not null, columns >= Nb/2 of the product go to

@@ -40,6 +40,9 @@ SIGNATURES = {
     "lewi_grouped_gemm_dh_dswiglu_scaled": (c_int, [P, P, P, P, P, P, P, P, P, P, P, c_int64, c_int, c_int, c_int]),
     "lewi_group_tables": (c_int, [P, P, c_int64, c_int, c_int, P, P, P, P, P]),
     "lewi_gather_rows": (c_int, [P, P, P, P, P, c_int64, c_int64, c_int, c_int, c_int, c_int, P, c_int]),
+    "lewi_ragged_gemm_ok": (c_int, [c_int64, c_int]),
+    "lewi_group_offsets": (c_int, [P, P, c_int, P]),
+    "lewi_ragged_gemm": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int]),
     "lewi_dispatch_tokens": (c_int, [P, P, P, P, c_int64, c_int, c_int, c_int]),
     "lewi_combine_bwd": (c_int, [P, P, P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int]),
     "lewi_dispatch_rows": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int64, P, c_int]),

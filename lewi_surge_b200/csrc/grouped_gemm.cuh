@@ -86,6 +86,8 @@ struct Args {
   const float* col_bias;        // PLAIN: optional f32 per output column
   const float* r1_row;          // PLAIN: optional rank-one term added to the product: out[r,n] += r1_row[r] * r1_col[n]
   const float* r1_col;
+  int compact;                  // pair kernels, NN / NT PLAIN with bf16 output: groups follow one another without padding (pad_offsets:
+                                // E+1 offsets of any alignment); rows past the last group are stored as zeros
   int skip_rows;                // pair kernels, NN / NT: experts of at most this many padded rows are left out
   int tn_part_rows;             // TN over several experts: > 0 cuts an expert's contraction into parts of this many rows
                                 // (a multiple of 64); experts with more than one part go through `partial`
@@ -166,6 +168,7 @@ struct Tile {
   int e;        // expert
   int second;   // pair mode, NN/NT: 1 if the second 128-row block of the pair belongs to the same expert
   int row0;     // first row of the row-indexed operand (NN/NT: A rows; TN: first contraction row)
+  long long row_end;   // NN/NT: end of the rows that this tile may store
   int m0;       // TN: first output row
   int n0;       // first accumulator column in output coordinates (SWIGLU: first h column)
   int nlim;     // columns >= nlim are not stored by this tile
@@ -174,12 +177,15 @@ struct Tile {
   int split;    // TN: slot of this part in `partial`, or -1 when the tile is stored straight to the output
 };
 
-// Row-block pairs (pair mode, NN/NT): expert e owns ceil(blocks_e / 2) pairs; pp[e] is the exclusive
-// prefix of those counts (uint16 in shared memory).  Pair p belongs to the largest e with pp[e] <= p.
+// Row-block pairs (pair mode, NN/NT): expert e owns ceil(rows_e / 256) pairs; pp[e] is the exclusive
+// prefix of those counts (uint16 in shared memory).  Pair p belongs to the largest e with pp[e] <= p.  Groups need not start on a
+// block: rows that follow one another without padding (compact) are loaded like any others, what a tile reads past its group's end is
+// the next group's and is not stored.
 template <int MAJOR, int EPI, bool PAIR>
 __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles_n, const uint16_t* pp) {
   Tile t;
   t.second = 1;
+  t.row_end = a.rows;
   if constexpr (MAJOR == TN) {
     constexpr int TM = PAIR ? 2 * BM : BM;
     const int m_tiles = (a.Ma + TM - 1) / TM;
@@ -250,9 +256,9 @@ __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles
           if ((int)pp[mid] <= unit) lo = mid; else hi = mid;
         }
         t.e = lo;
-        const int first = a.pad_offsets[lo] / BM + 2 * (unit - (int)pp[lo]);
-        t.row0 = first * BM;
-        t.second = (first + 1) * BM < a.pad_offsets[lo + 1];
+        t.row0 = a.pad_offsets[lo] + (unit - (int)pp[lo]) * 2 * BM;
+        t.row_end = min(a.rows, (long long)a.pad_offsets[lo + 1]);
+        t.second = (long long)t.row0 + BM < t.row_end;
       } else {
         t.e = 0;
         t.row0 = unit * 2 * BM;
@@ -366,8 +372,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     if (a.tn_part_rows > 0 && warp == 1)
       expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return max(1, (rows_e + a.tn_part_rows - 1) / a.tn_part_rows); });
   } else if constexpr (PAIR) {
-    // exclusive prefix of ceil(blocks_e / 2)
-    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return rows_e > a.skip_rows ? (rows_e / BM + 1) >> 1 : 0; });
+    // exclusive prefix of ceil(rows_e / 256)
+    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return rows_e > a.skip_rows ? (rows_e + 2 * BM - 1) / (2 * BM) : 0; });
   }
   if (warp == 1) {
     if constexpr (PAIR) {
@@ -535,12 +541,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     [[maybe_unused]] uint32_t epi_phase = 0;
     [[maybe_unused]] TileStager<staging_tiles(EPI)> out2buf{stage, 0};
     bool ok = true;
+    if constexpr (EPI == PLAIN && PAIR) {
+      if (a.compact) {
+        const long long last = a.pad_offsets[a.E];
+        if (last > a.rows && blockIdx.x == 0 && threadIdx.x == 64) raise_status(LEWI_STATUS_BAD_INDEX);
+        for (long long r = last + blockIdx.x * EPI_WARPS + (warp - 2); r < a.rows; r += (long long)gridDim.x * EPI_WARPS)
+          for (int n = lane * 8; n < a.N; n += 256) st_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + r * a.N + n, make_uint4(0, 0, 0, 0));
+      }
+    }
     for (int tile = tile_first; ok && tile < total_tiles; tile += tile_step) {
       const Tile t = decode_tile<MAJOR, EPI, PAIR>(a, tile, n_tiles_n, pair_prefix);
       const bool has_acc = t.kb > 0;
       // first row (of the output tensor) handled by this warp and how many of its 32 rows exist
       const long long wrow0 = (MAJOR == TN ? (long long)t.m0 : (long long)t.row0) + (long long)cta_rank * BM + lane_grp * 32;
-      const long long row_lim = MAJOR == TN ? (long long)a.Ma : a.rows;
+      const long long row_lim = MAJOR == TN ? (long long)a.Ma : t.row_end;
       int rows_valid = (int)max(0LL, min(32LL, row_lim - wrow0));
       if (MAJOR != TN && cta_rank == 1 && !t.second) rows_valid = 0;   // this CTA's block belongs to the next expert
       const int n_end = t.nlim;
@@ -651,7 +665,20 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
               if ((c & 1) == 0) buf = out2buf.acquire(lane);
               tile_put_bf16x32(buf, lane, (c & 1) * 4, v);
               // a 64-column tile is complete after its odd 32-column block, or when the row ends inside it
-              if ((c & 1) == 1 || n + 32 >= n_end) out2buf.store2d(lane, &tm_c, buf, n - (c & 1) * 32, (int)wrow0);
+              if ((c & 1) == 1 || n + 32 >= n_end) {
+                if (a.compact && rows_valid < 32) {   // the rows below belong to the next group
+                  __syncwarp();
+                  const int piece = lane & 7, nb = n - (c & 1) * 32;
+#pragma unroll 1
+                  for (int row = lane >> 3; row < rows_valid; row += 4)
+                    if (nb + piece * 8 < a.N)
+                      st_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + (wrow0 + row) * a.N + nb + piece * 8,
+                            *reinterpret_cast<const uint4*>(buf + row * 128 + ((piece ^ (row & 7)) << 4)));
+                  __syncwarp();
+                } else {
+                  out2buf.store2d(lane, &tm_c, buf, n - (c & 1) * 32, (int)wrow0);
+                }
+              }
             }
           }
         }

@@ -426,6 +426,7 @@ inline void fill_common(gg::Args& a, const RowGroupArgs& r) {
   a.col_bias = nullptr;
   a.r1_row = nullptr;
   a.r1_col = nullptr;
+  a.compact = 0;
   a.skip_rows = r.skip_rows;
   a.tn_part_rows = 0;
   a.scale_src = nullptr;
@@ -708,6 +709,47 @@ int lewi_grouped_gemm_nt(void* stream, const void* a_ptr, const void* b_ptr, voi
   if (!gg::make_out_map(&tc, out, (uint64_t)N, (uint64_t)rows, 0, a.out_f32 != 0)) return LEWI_ERR_CUDA;
   const long long tiles = (long long)a.n_blocks_host * ((N + gg::BN - 1) / gg::BN);
   return gg::launch_auto<gg::NT, gg::PLAIN>(pair, as_stream(stream), ta, tb, tb, a, tiles, &tc);
+}
+
+namespace {
+inline bool ragged_ok(int64_t m, int E) {   // (pair prefixes are kept as 16-bit counts)
+  return gg::pair_mode() && E > 0 && E <= kMaxExperts && m >= 0 && m <= 0x7fffff00LL && m / (2 * gg::BM) + E + 1 < 65535;
+}
+}  // namespace
+
+int lewi_ragged_gemm_ok(int64_t m, int E) { return ragged_ok(m, E) ? 1 : 0; }
+
+int lewi_group_offsets(void* stream, const int32_t* group_sizes, int E, int32_t* offsets) {
+  if (!group_sizes || !offsets || E <= 0) return LEWI_ERR_ARG;
+  if (E > kMaxExperts) return LEWI_ERR_LIMIT;
+  group_offsets_kernel<<<1, kRouteThreads, 0, as_stream(stream)>>>(group_sizes, E, offsets);
+  LEWI_CHECK_LAUNCH();
+  return LEWI_OK;
+}
+
+int lewi_ragged_gemm(void* stream, const void* a_ptr, const void* b_ptr, void* out, const int32_t* offsets, int64_t m, int K, int N, int E,
+                     int transposed) {
+  if (!a_ptr || !b_ptr || !out || !offsets || K <= 0 || N <= 0 || E <= 0 || m < 0) return LEWI_ERR_ARG;
+  if (!ragged_ok(m, E)) return LEWI_ERR_LIMIT;
+  if (K % 8 != 0 || N % 8 != 0 || !aligned16(a_ptr) || !aligned16(b_ptr) || !aligned16(out)) return LEWI_ERR_SHAPE;
+  if (m == 0) return LEWI_OK;
+  CUtensorMap ta, tb, tc;
+  if (!gg::make_map(&ta, a_ptr, (uint64_t)K, (uint64_t)m, 0, 64, 128) || !gg::make_out_map(&tc, out, (uint64_t)N, (uint64_t)m, 0, false) ||
+      !(transposed ? gg::make_map(&tb, b_ptr, (uint64_t)K, (uint64_t)N, (uint64_t)E, 64, 128)
+                   : gg::make_map(&tb, b_ptr, (uint64_t)N, (uint64_t)K, (uint64_t)E, 64, 64)))
+    return LEWI_ERR_CUDA;
+  RowGroupArgs r{nullptr, nullptr, offsets, m, E};
+  gg::Args a;
+  fill_common(a, r);
+  a.n_blocks_host = (int)(m / (2 * gg::BM) + E);   // bound on the groups' pairs of row blocks
+  a.compact = 1;
+  a.out = out;
+  a.K = K;
+  a.kb_total = (K + gg::BK - 1) / gg::BK;
+  a.N = N;
+  const long long tiles = (long long)a.n_blocks_host * ((N + gg::BN - 1) / gg::BN);
+  if (transposed) return gg::launch_auto<gg::NT, gg::PLAIN>(true, as_stream(stream), ta, tb, tb, a, tiles, &tc);
+  return gg::launch_auto<gg::NN, gg::PLAIN>(true, as_stream(stream), ta, tb, tb, a, tiles, &tc);
 }
 
 namespace {

@@ -719,6 +719,15 @@ __global__ void __launch_bounds__(kRouteThreads) group_tables_kernel(const int32
 }
 
 // f32 -> bf16 (round to nearest even), grid-stride.
+// offsets[e] = sum of the sizes of the groups before e (negative sizes count as none), e in [0, E].
+__global__ void __launch_bounds__(kRouteThreads) group_offsets_kernel(const int32_t* __restrict__ gs, int E, int32_t* __restrict__ offsets) {
+  __shared__ int s_cnt[kMaxExperts], s_off[kMaxExperts + 1], s_pad[kMaxExperts + 1], s_tmp[2 * kRouteWarps];
+  if (threadIdx.x < E) s_cnt[threadIdx.x] = max(gs[threadIdx.x], 0);
+  __syncthreads();
+  expert_offsets(s_cnt, E, 0, s_off, s_pad, s_tmp, threadIdx.x);
+  for (int x = threadIdx.x; x <= E; x += kRouteThreads) offsets[x] = s_off[x];
+}
+
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ src,
                                                             __nv_bfloat16* __restrict__ dst, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)

@@ -326,8 +326,20 @@ def grouped_gemm_tn(a, b, pad_offsets, num_experts, out_dtype=torch.bfloat16, ou
   return (out, out2) if split else out
 
 
+def _ragged_gemm(a, b, offsets, transposed):
+  """rows of a (M, K), sorted by group and not padded, times their group's matrix: b (E, K, N), or (E, N, K) transposed."""
+  lib = _lib.load()
+  (m, k), e = a.shape, b.shape[0]
+  n = b.shape[1 if transposed else 2]
+  out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
+  check(lib.lewi_ragged_gemm(stream(), ptr(a), ptr(b), ptr(out), ptr(offsets), m, k, n, e, int(transposed)), "lewi_ragged_gemm")
+  return out
+
+
 class _RaggedDot(torch.autograd.Function):
-  """Dropless grouped GEMM with the reference's gather -> batched GEMM -> gather structure.
+  """Dropless grouped GEMM.  The products over rows run on the rows as they come (gathered into padded groups and back they took two
+  passes over them each: 36,006 rows over 64 groups, 1024 x 512, forward 94 -> 52 us); the weight gradient contracts over rows and reads
+  them gathered into padded groups.
 
   Reference: padded_ragged_dot, modal/padded_gmm.py:45-69 (and te_ragged_dot, modal/te_gmm.py:12-19
   for the dropless semantics): rows of lhs are sorted by expert, group g multiplies rhs[g], rows past
@@ -336,26 +348,39 @@ class _RaggedDot(torch.autograd.Function):
 
   @staticmethod
   def forward(ctx, lhs, rhs, group_sizes):
-    m, _ = lhs.shape
-    e = rhs.shape[0]
-    t = group_tables(group_sizes, m)
+    lib = _lib.load()
+    m, k = lhs.shape
+    e, n = rhs.shape[0], rhs.shape[2]
     a = lhs.to(torch.bfloat16).contiguous()
     b = rhs.to(torch.bfloat16).contiguous()
+    ctx.e, ctx.lhs_dtype, ctx.rhs_dtype = e, lhs.dtype, rhs.dtype
+    ctx.compact = 0 < m and max(k, n) <= 4096 and lib.lewi_ragged_gemm_ok(m, e) == 1   # (rows beyond 4096 cannot be gathered for the gradient)
+    if ctx.compact:
+      gs = _i32(group_sizes).contiguous()
+      offsets = torch.empty(e + 1, dtype=torch.int32, device=gs.device)
+      check(lib.lewi_group_offsets(stream(), ptr(gs), e, ptr(offsets)), "lewi_group_offsets")
+      ctx.save_for_backward(a, b, gs, offsets)
+      return _ragged_gemm(a, b, offsets, False).to(lhs.dtype)
+    t = group_tables(group_sizes, m)
     buf = gather_rows(a, t["row_of_padded"])
     out_pad = grouped_gemm_nn(buf, b, t["block_expert"], t["n_blocks"], pad_offsets=t["pad_offsets"])
     out = gather_rows(out_pad, t["padded_of_row"])
     ctx.save_for_backward(buf, b, t["row_of_padded"], t["padded_of_row"], t["block_expert"], t["n_blocks"],
                           t["pad_offsets"])
-    ctx.e, ctx.lhs_dtype, ctx.rhs_dtype = e, lhs.dtype, rhs.dtype
     return out.to(lhs.dtype)
 
   @staticmethod
   def backward(ctx, g):
-    buf, b, row_of_padded, padded_of_row, block_expert, n_blocks, pad_offsets = ctx.saved_tensors
-    g_pad = gather_rows(g.to(torch.bfloat16).contiguous(), row_of_padded)
-    # dlhs = g . rhs[e]^T: rhs [E,K,N] read as the K-major operand with contraction over N
-    dl_pad = grouped_gemm_nt(g_pad, b, block_expert, n_blocks, pad_offsets=pad_offsets)
-    dlhs = gather_rows(dl_pad, padded_of_row)
+    g = g.to(torch.bfloat16).contiguous()
+    if ctx.compact:
+      a, b, gs, offsets = ctx.saved_tensors
+      dlhs = _ragged_gemm(g, b, offsets, True)   # g . rhs[e]^T: rhs [E,K,N] read as the K-major operand with contraction over N
+      t = group_tables(gs, a.shape[0])
+      buf, g_pad, pad_offsets = gather_rows(a, t["row_of_padded"]), gather_rows(g, t["row_of_padded"]), t["pad_offsets"]
+    else:
+      buf, b, row_of_padded, padded_of_row, block_expert, n_blocks, pad_offsets = ctx.saved_tensors
+      g_pad = gather_rows(g, row_of_padded)
+      dlhs = gather_rows(grouped_gemm_nt(g_pad, b, block_expert, n_blocks, pad_offsets=pad_offsets), padded_of_row)
     # rounded once from the float32 accumulators where the weights are bf16
     drhs = grouped_gemm_tn(buf, g_pad, pad_offsets, ctx.e, out_dtype=torch.bfloat16 if ctx.rhs_dtype == torch.bfloat16 else torch.float32)
     return dlhs.to(ctx.lhs_dtype), drhs.to(ctx.rhs_dtype), None

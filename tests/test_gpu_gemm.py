@@ -345,3 +345,41 @@ def test_parts_of_heavy_experts_are_summed_wherever_they_stand(cuda, e, heavy, s
   for x in range(e):
     want = a[pads[x]:pads[x + 1]].float().T @ b[pads[x]:pads[x + 1]].float()
     assert torch.equal(got[x], want), x
+
+
+@pytest.mark.parametrize("sizes,tail,k,n,dt", [((5, 0, 9, 3, 7, 1, 6, 4), 3, 64, 48, "bf16"), ((1,), 0, 8, 8, "bf16"), ((257, 0, 255, 256, 1, 31), 40, 136, 264, "bf16"),
+                                               ((0, 0, 0), 5, 64, 64, "bf16"), ((33,) * 130, 1, 72, 520, "f32"), ((300, 700, 20), -100, 128, 256, "bf16")])
+def test_ragged_products_on_unpadded_rows_equal_the_padded_ones(cuda, monkeypatch, sizes, tail, k, n, dt):
+  """Groups that start and end anywhere, empty ones, rows past the last (tail < 0: groups that ask for more rows than there are, of which
+  those within are compared).  Same bits as with padding, out and both gradients; an infinite row reaches no other group."""
+  from lewi_surge_b200 import ops, _lib
+  lib, e, m = _lib.load(), len(sizes), sum(sizes) + tail
+  gen = torch.Generator(device=cuda).manual_seed(m)
+  dtype = torch.float32 if dt == "f32" else torch.bfloat16
+  rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda).to(dtype)
+  gs = torch.tensor(sizes, dtype=torch.int32, device=cuda)
+  lhs, rhs, g = rnd(m, k), rnd(e, k, n), rnd(m, n)
+  first = next((i for i, v in enumerate(sizes) if v > 0), None)
+  if tail >= 0 and first is not None and e > 1:
+    lhs[0, 0] = float("inf")
+  def run():
+    a, b = lhs.clone().requires_grad_(True), rhs.clone().requires_grad_(True)
+    out = ops.ragged_dot(a, b, gs)
+    return out.detach(), *torch.autograd.grad(out, (a, b), g)
+  _lib.last_status()
+  got = run()
+  status = _lib.last_status()
+  assert (status != 0) == (tail < 0)   # the status says that rows are missing
+  if tail < 0:
+    for x, lo in enumerate(np.concatenate([[0], np.cumsum(sizes)[:-1]])):
+      want = lhs[lo:lo + sizes[x]].float() @ rhs[x].float()
+      assert O.rel_err(to_np(got[0][lo:lo + sizes[x]].float()), to_np(want)) <= 1e-2
+    return
+  monkeypatch.setattr(lib, "lewi_ragged_gemm_ok", lambda m_, e_: 0)
+  want = run()
+  assert _lib.last_status() == 0
+  for x, y in zip(got, want):
+    assert torch.equal(torch.nan_to_num(x.float(), nan=1e30), torch.nan_to_num(y.float(), nan=1e30))
+  assert not got[0][m - tail:].any() and not got[1][m - tail:].any()
+  if first is not None and e > 1:
+    assert got[0][sizes[first]:].isfinite().all() and got[2][first + 1:].isfinite().all()
