@@ -364,7 +364,9 @@ def test_ragged_products_on_unpadded_rows_equal_the_padded_ones(cuda, monkeypatc
     lhs[0, 0] = float("inf")
   def run():
     a, b = lhs.clone().requires_grad_(True), rhs.clone().requires_grad_(True)
-    out = ops.ragged_dot(a, b, gs)
+    mine = gs.clone()
+    out = ops.ragged_dot(a, b, mine)
+    mine.zero_()   # the caller's buffer for the next call
     return out.detach(), *torch.autograd.grad(out, (a, b), g)
   _lib.last_status()
   got = run()
