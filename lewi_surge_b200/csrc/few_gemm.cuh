@@ -62,6 +62,9 @@ struct Args {
   const float* col_bias;         // LOGITS: f32 [N] or null
   uint64_t desc_hi_w, desc_hi_r;
   uint32_t idesc;                // without N
+  // Launched early (common.cuh): only the rows are waited for, since the weights and the routing tables are older than the kernel before
+  // this one, which had itself waited for them when it let this one start; otherwise everything is.
+  int rows_only;
 };
 
 struct Tile {
@@ -144,6 +147,10 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (!a.rows_only) {
+    grid_wait();
+    grid_launch();   // (after the wait: what starts now may count on everything before THIS kernel)
+  }
   const int n_units = a.n_blocks != nullptr ? min(a.units, max(a.n_blocks[0], 0)) : a.units;
   const int total = n_units * a.n_tiles, step = (int)gridDim.x;
 
@@ -219,6 +226,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
     // ------------------------------------------------------------------ rows
     const int ld = warp < 4 ? warp - 2 : warp - 6;
     const int stages_per_tile = (a.kb_total + KPS - 1) / KPS;
+    grid_wait();
     uint32_t it0 = 0;
     Tile next = decode<EPI>(a, blockIdx.x, total);
     for (int tile = blockIdx.x; tile < total; tile += step) {
@@ -270,6 +278,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
   } else {
     // ------------------------------------------------------------------ epilogue
     const int tid = threadIdx.x - 128, grp = warp & 3;
+    grid_wait();
     uint32_t acc_it = 0;
     Tile next = decode<EPI>(a, blockIdx.x, total);
     for (int tile = blockIdx.x; tile < total; tile += step) {
@@ -366,7 +375,7 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
 }
 
 template <int EPI>
-inline int launch(cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tr, Args a, int max_rows) {
+inline int launch(cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tr, Args a, int max_rows, bool early = false) {
   static bool attr_set[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return LEWI_ERR_CUDA;
@@ -395,7 +404,7 @@ inline int launch(cudaStream_t st, const CUtensorMap& tw, const CUtensorMap& tw2
   if (gg::cta_limit() > 0 && grid > gg::cta_limit()) grid = gg::cta_limit();
   if (grid > tiles) grid = tiles;
   const int smem = a.stages * a.stage_bytes + STAGING_BYTES + BAR_BYTES;
-  kern<<<(int)grid, THREADS, smem, st>>>(tw, tw2, tr, a);
+  (void)launch_kernel(kern, (int)grid, THREADS, (size_t)smem, st, early, tw, tw2, tr, a);
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }

@@ -223,6 +223,8 @@ __global__ void __launch_bounds__(kRouteThreads) route_chunk_kernel(RouteChunkAr
   const int n_slots = (int)min((long long)a.chunk_slots, a.num_slots - slot0);
 
   for (int i = tid; i < a.E; i += kRouteThreads) s_hist[i] = 0;
+  grid_wait();
+  grid_launch();
   if (a.row_slot != nullptr) {
     for (long long r = (long long)blockIdx.x * kRouteThreads + tid; r < a.mpad; r += (long long)gridDim.x * kRouteThreads)
       a.row_slot[r] = -1;
@@ -441,6 +443,8 @@ __global__ void __launch_bounds__(kRouteThreads) route_rank_kernel(RouteRankArgs
     s_cnt[e] = 0;
     s_base[e] = 0;
   }
+  grid_wait();
+  grid_launch();
   for (int i = tid; i < n_slots; i += kRouteThreads) {
     const int e = a.flat[slot0 + i];
     s_e[i] = (e < 0 || e >= E) ? -1 : e;
@@ -511,6 +515,8 @@ __global__ void __launch_bounds__(kRouteThreads) route_fused_kernel(RouteFusedAr
   int* s_run = s_mem + (n_slots + 3) / 4 * 4;   // [kRouteWarps][E], the column sums of the soft-max before that
   float* s_prob = reinterpret_cast<float*>(s_run);
   for (int e = tid; e < E; e += kRouteThreads) s_cnt[e] = 0;
+  grid_wait();
+  grid_launch();
   if (a.t.row_slot != nullptr)
     for (long long r = tid; r < a.mpad; r += kRouteThreads) a.t.row_slot[r] = -1;
   route_chunk_tokens<ER>(a.logits, a.topk_idx, a.topk_w, 0, n_slots / a.k, E, a.k, s_e, s_prob, a.t.probs_sum != nullptr, lane, warp);
@@ -785,21 +791,21 @@ inline bool route_smem_ok(Kern kern, size_t smem, bool (&done)[64]) {
 }
 
 template <int ER>
-inline int launch_route_chunk(cudaStream_t st, const RouteChunkArgs& a, int n_chunks) {
+inline int launch_route_chunk(cudaStream_t st, const RouteChunkArgs& a, int n_chunks, bool early) {
   static bool done[64] = {false};
   const size_t smem = ((size_t)a.chunk_slots + (size_t)(kRouteWarps + 1) * a.E) * 4;
   if (!route_smem_ok(route_chunk_kernel<ER>, smem, done)) return LEWI_ERR_LIMIT;
-  route_chunk_kernel<ER><<<n_chunks, kRouteThreads, smem, st>>>(a);
+  (void)launch_kernel(route_chunk_kernel<ER>, n_chunks, kRouteThreads, smem, st, early, a);
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }
 
 template <int ER>
-inline int launch_route_fused(cudaStream_t st, const RouteFusedArgs& a) {
+inline int launch_route_fused(cudaStream_t st, const RouteFusedArgs& a, bool early) {
   static bool done[64] = {false};
   const size_t smem = ((size_t)a.t.num_slots + 4 + (size_t)kRouteWarps * a.t.E) * 4;
   if (!route_smem_ok(route_fused_kernel<ER>, smem, done)) return LEWI_ERR_LIMIT;
-  route_fused_kernel<ER><<<1, kRouteThreads, smem, st>>>(a);
+  (void)launch_kernel(route_fused_kernel<ER>, 1, kRouteThreads, smem, st, early, a);
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }
@@ -808,7 +814,7 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
                         int E, int k, int block, int32_t* topk_idx, float* topk_w, int32_t* counts,
                         int32_t* offsets, int32_t* pad_offsets, int32_t* block_expert, int32_t* n_blocks,
                         int32_t* order, int32_t* pos, int32_t* pad_pos, int32_t* row_slot, float* probs_sum,
-                        void* ws, long long ws_bytes, float* aux_loss = nullptr) {
+                        void* ws, long long ws_bytes, float* aux_loss = nullptr, bool early = false) {
   if (E <= 0 || E > kMaxExperts) return LEWI_ERR_LIMIT;
   if (M > 0x7fffffffLL) return LEWI_ERR_LIMIT;
   const bool padded = block > 0 && pad_offsets != nullptr;
@@ -846,7 +852,7 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
   if (ws == nullptr || ws_bytes < need) return LEWI_ERR_WORKSPACE;   // also where the one-CTA path would not touch it
   if (logits != nullptr && route_fused(T, E, n_chunks)) {
     const RouteFusedArgs fa{t, logits, topk_idx, topk_w, mpad, k};
-    LEWI_ROUTE_ER(launch_route_fused<ER>(st, fa));
+    LEWI_ROUTE_ER(launch_route_fused<ER>(st, fa, early));
     return LEWI_OK;
   }
   int32_t* chunk_hist = reinterpret_cast<int32_t*>(ws);
@@ -866,8 +872,8 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
   ca.chunk_slots = chunk_slots;
   if (n_chunks > 0) {
     if (logits) {
-      LEWI_ROUTE_ER(launch_route_chunk<ER>(st, ca, n_chunks));
-    } else if (int rc = launch_route_chunk<1>(st, ca, n_chunks)) {
+      LEWI_ROUTE_ER(launch_route_chunk<ER>(st, ca, n_chunks, early));
+    } else if (int rc = launch_route_chunk<1>(st, ca, n_chunks, early)) {
       return rc;
     }
   } else if (padded && row_slot != nullptr && mpad > 0) {
@@ -883,7 +889,7 @@ inline int route_common(cudaStream_t st, const float* logits, const int32_t* fla
   // s_run [kRouteWarps][E] also holds one partial probability sum per thread
   const size_t smem = ((size_t)chunk_slots + (size_t)(kRouteWarps * E > kRouteThreads ? kRouteWarps * E : kRouteThreads)) * 4;
   if (!route_smem_ok(route_rank_kernel, smem, done)) return LEWI_ERR_LIMIT;
-  route_rank_kernel<<<n_chunks > 0 ? n_chunks : 1, kRouteThreads, smem, st>>>(ra);
+  (void)launch_kernel(route_rank_kernel, n_chunks > 0 ? n_chunks : 1, kRouteThreads, smem, st, early && !scanned && n_chunks > 0, ra);
   LEWI_CHECK_LAUNCH();
   return LEWI_OK;
 }
