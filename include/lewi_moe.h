@@ -235,8 +235,10 @@ int lewi_grouped_gemm_nt(void* stream, const void* a, const void* b, void* out, 
 
 /* `jax.lax.ragged_dot` (modal/padded_gmm.py:45) on rows as they come, sorted by group and without padding: out[r] = a[r] . b[e] for
  * offsets[e] <= r < offsets[e+1], zeros for r >= offsets[E]; a bf16 [m,K], out bf16 [m,N], b bf16 [E,K,N], or [E,N,K] with transposed.
- * offsets i32 [E+1] on the device, as lewi_group_offsets writes them.  lewi_ragged_gemm_ok: 1 where it can be used (CTA pairs not
- * switched off, sizes within their tables); otherwise pad the rows (lewi_group_tables). */
+ * offsets i32 [E+1] on the device, as lewi_group_offsets writes them (sums of the sizes, held at 2^31 - 1 beyond).  Offsets that leave
+ * [0, m] or fall raise LEWI_STATUS_BAD_INDEX and nothing outside out is written; where none falls, groups within [0, m] have their rows.
+ * lewi_ragged_gemm_ok: 1 where it can be used (CTA pairs not switched off, sizes within their tables); otherwise pad the rows
+ * (lewi_group_tables). */
 int lewi_ragged_gemm_ok(int64_t m, int E);
 int lewi_group_offsets(void* stream, const int32_t* group_sizes, int E, int32_t* offsets);
 int lewi_ragged_gemm(void* stream, const void* a, const void* b, void* out, const int32_t* offsets, int64_t m, int K, int N, int E,

@@ -177,6 +177,14 @@ struct Tile {
   int split;    // TN: slot of this part in `partial`, or -1 when the tile is stored straight to the output
 };
 
+// Rows [lo, hi) of the tensor that a group of the pair kernels (NN / NT) has by its offsets.  Offsets that lie outside the tensor or fall (a
+// table gone wrong) name no rows beyond it: every row that is stored lies in [0, rows).
+__device__ __forceinline__ int2 rows_of_group(const Args& a, int lo, int hi) {
+  const int n = (int)min(a.rows, 0x7fffffffLL);
+  const int first = min(max(lo, 0), n);
+  return make_int2(first, min(max(hi, first), n));
+}
+
 // Row-block pairs (pair mode, NN/NT): expert e owns ceil(rows_e / 256) pairs; pp[e] is the exclusive
 // prefix of those counts (uint16 in shared memory).  Pair p belongs to the largest e with pp[e] <= p.  Groups need not start on a
 // block: rows that follow one another without padding (compact) are loaded like any others, what a tile reads past its group's end is
@@ -256,8 +264,11 @@ __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles
           if ((int)pp[mid] <= unit) lo = mid; else hi = mid;
         }
         t.e = lo;
-        t.row0 = a.pad_offsets[lo] + (unit - (int)pp[lo]) * 2 * BM;
-        t.row_end = min(a.rows, (long long)a.pad_offsets[lo + 1]);
+        const int2 r = rows_of_group(a, a.pad_offsets[lo], a.pad_offsets[lo + 1]);
+        const long long first = r.x + (unit - (long long)pp[lo]) * 2 * BM;
+        const bool in = first >= r.x && first < r.y;   // (else the groups overlap and have more pairs than 16 bits count: nothing is stored)
+        t.row0 = in ? (int)first : r.x;
+        t.row_end = in ? r.y : r.x;
         t.second = (long long)t.row0 + BM < t.row_end;
       } else {
         t.e = 0;
@@ -276,7 +287,7 @@ __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles
   return t;
 }
 
-// prefix[e] = sum over x < e of count(rows of expert x), e in [0, E], by one warp: all offsets are requested at once and
+// prefix[e] = sum over x < e of count(offsets of expert x), e in [0, E], by one warp: all offsets are requested at once and
 // scanned with shuffles.  (One thread that walked them took 8 us at 128 experts, before the first tile of every GEMM.)
 template <class F>
 __device__ __forceinline__ void expert_prefix(uint16_t* prefix, const int32_t* __restrict__ pad_offsets, int E, int lane, F count) {
@@ -292,7 +303,7 @@ __device__ __forceinline__ void expert_prefix(uint16_t* prefix, const int32_t* _
 #pragma unroll
   for (int x = 0; x < NV; ++x) {
     if (x * 32 >= E) break;
-    const int e = x * 32 + lane, c = e < E ? count(hi[x] - lo[x]) : 0;
+    const int e = x * 32 + lane, c = e < E ? count(lo[x], hi[x]) : 0;
     int run = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -370,10 +381,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
   if constexpr (MAJOR == TN) {
     // exclusive prefix of the experts' contraction-part counts
     if (a.tn_part_rows > 0 && warp == 1)
-      expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return max(1, (rows_e + a.tn_part_rows - 1) / a.tn_part_rows); });
+      expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int lo, int hi) { return max(1, (hi - lo + a.tn_part_rows - 1) / a.tn_part_rows); });
   } else if constexpr (PAIR) {
     // exclusive prefix of ceil(rows_e / 256)
-    if (a.pad_offsets != nullptr && warp == 1) expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int rows_e) { return rows_e > a.skip_rows ? (rows_e + 2 * BM - 1) / (2 * BM) : 0; });
+    if (a.pad_offsets != nullptr && warp == 1)
+      expert_prefix(pair_prefix, a.pad_offsets, a.E, lane, [&](int lo, int hi) {
+        const int2 r = rows_of_group(a, lo, hi);
+        if (a.compact && (r.x != lo || r.y != hi) && blockIdx.x == 0) raise_status(LEWI_STATUS_BAD_INDEX);
+        return r.y - r.x > a.skip_rows ? (r.y - r.x + 2 * BM - 1) / (2 * BM) : 0;
+      });
   }
   if (warp == 1) {
     if constexpr (PAIR) {
@@ -543,8 +559,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     bool ok = true;
     if constexpr (EPI == PLAIN && PAIR) {
       if (a.compact) {
-        const long long last = a.pad_offsets[a.E];
-        if (last > a.rows && blockIdx.x == 0 && threadIdx.x == 64) raise_status(LEWI_STATUS_BAD_INDEX);
+        const long long last = rows_of_group(a, a.pad_offsets[a.E - 1], a.pad_offsets[a.E]).y;
         for (long long r = last + blockIdx.x * EPI_WARPS + (warp - 2); r < a.rows; r += (long long)gridDim.x * EPI_WARPS)
           for (int n = lane * 8; n < a.N; n += 256) st_v4(reinterpret_cast<__nv_bfloat16*>(a.out) + r * a.N + n, make_uint4(0, 0, 0, 0));
       }

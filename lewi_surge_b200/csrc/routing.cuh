@@ -724,16 +724,27 @@ __global__ void __launch_bounds__(kRouteThreads) group_tables_kernel(const int32
   }
 }
 
-// f32 -> bf16 (round to nearest even), grid-stride.
-// offsets[e] = sum of the sizes of the groups before e (negative sizes count as none), e in [0, E].
+// offsets[e] = sum of the sizes of the groups before e (negative sizes count as none), e in [0, E]; sums beyond 2^31 - 1 stay there, so that
+// the offsets never fall.
 __global__ void __launch_bounds__(kRouteThreads) group_offsets_kernel(const int32_t* __restrict__ gs, int E, int32_t* __restrict__ offsets) {
-  __shared__ int s_cnt[kMaxExperts], s_off[kMaxExperts + 1], s_pad[kMaxExperts + 1], s_tmp[2 * kRouteWarps];
-  if (threadIdx.x < E) s_cnt[threadIdx.x] = max(gs[threadIdx.x], 0);
+  __shared__ int s_sum[kRouteWarps];
+  static_assert(kMaxExperts <= kRouteThreads, "one expert per thread");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto add = [](int a, int b) { return (int)min((unsigned)a + (unsigned)b, 0x7fffffffu); };
+  int run = tid < E ? max(gs[tid], 0) : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run = add(run, up);
+  }
+  if (lane == 31) s_sum[warp] = run;
   __syncthreads();
-  expert_offsets(s_cnt, E, 0, s_off, s_pad, s_tmp, threadIdx.x);
-  for (int x = threadIdx.x; x <= E; x += kRouteThreads) offsets[x] = s_off[x];
+  for (int w = 0; w < warp; ++w) run = add(run, s_sum[w]);
+  if (tid < E) offsets[tid + 1] = run;
+  if (tid == 0) offsets[0] = 0;
 }
 
+// f32 -> bf16 (round to nearest even), grid-stride.
 __global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ src,
                                                             __nv_bfloat16* __restrict__ dst, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
