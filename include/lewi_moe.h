@@ -370,7 +370,8 @@ int lewi_gdn_chunk_bwd(void* stream, const void* q, const void* k, const void* v
  * side_stream (may be null or equal to stream): the shared expert, which needs only x / dout, and the forward pass's
  * experts of many rows beside those of few, are queued there
  * between two events so that it overlaps the memory-bound routing, dispatch and gather kernels; the call
- * returns with `stream` waiting for it.  The events per device are created on first use and kept.
+ * returns with `stream` waiting for it.  Each call holds events of its own while it
+ * queues (a few sets per device are created on first use and kept), so calls of several host threads may overlap.
  *
  * router_prepared (may be null): the bf16 pieces of w_router that the router GEMMs read, as written by
  * lewi_moe_prepare_router (lewi_moe_router_prepared_bytes(d,E) bytes); pass it to skip that conversion in

@@ -9,6 +9,7 @@
 #include "router_gemm.cuh"
 #include "routing.cuh"
 #include "seqmix.cuh"
+#include "stream_events.h"
 #include "gdn_bwd.cuh"
 
 #include <cstring>
@@ -1513,8 +1514,8 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
   // few rows per expert: the kernels of few_gemm.cuh; with more than a few blocks' worth of tokens only for experts of one block
   const bool heavy = T > moe::kFewTokens, few = moe::few_routed(T, D.M, E) && (!heavy || gg::pair_mode());
   const bool fork = (shared || (few && heavy)) && side_stream != nullptr && side_stream != stream;
-  moe::Events* ev = fork ? moe::events() : nullptr;
-  if (fork && ev == nullptr) return LEWI_ERR_CUDA;
+  const EventLease ev(fork);
+  if (fork && !ev.ok()) return LEWI_ERR_CUDA;
   void* sh_stream = fork ? side_stream : stream;
 
   float* logits = reinterpret_cast<float*>(res(LEWI_MOE_RES_LOGITS));
@@ -1530,8 +1531,7 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
 
   // the shared expert needs only x: on the side stream it runs beside the memory-bound routing and dispatch
   if (fork) {
-    if (cudaEventRecord(ev->fork_fwd, st) != cudaSuccess || cudaStreamWaitEvent(sd, ev->fork_fwd, 0) != cudaSuccess)
-      return LEWI_ERR_CUDA;
+    if (!stream_after(ev->fork, st, sd)) return LEWI_ERR_CUDA;
     moe::mark("side_begin", sh_stream);
   }
   auto shared_fwd = [&]() -> int {
@@ -1592,8 +1592,7 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
   if (few) {
     const int32_t* counts = reinterpret_cast<const int32_t*>(res(LEWI_MOE_RES_COUNTS));
     if (heavy) {   // experts of several blocks go through the pair kernels, beside the others where there is a side stream
-      if (fork && (cudaEventRecord(ev->routed_fwd, st) != cudaSuccess || cudaStreamWaitEvent(sd, ev->routed_fwd, 0) != cudaSuccess))
-        return LEWI_ERR_CUDA;
+      if (fork && !stream_after(ev->mid, st, sd)) return LEWI_ERR_CUDA;
       const int max_blocks = (int)(D.Mpad / moe::kBlock);
       const int units = max_blocks * (moe::kBlock / kHeavyRows);
       gather_heavy_kernel<<<units < 4 * num_sms() ? units : 4 * num_sms(), 256, 0, as_stream(sh_stream)>>>(
@@ -1631,8 +1630,7 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
   }
   if (shared && !fork) LEWI_TRY(shared_fwd());
   if (fork) {
-    if (cudaEventRecord(ev->join_fwd, sd) != cudaSuccess || cudaStreamWaitEvent(st, ev->join_fwd, 0) != cudaSuccess)
-      return LEWI_ERR_CUDA;
+    if (!stream_after(ev->join, sd, st)) return LEWI_ERR_CUDA;
   }
   // combine: out[t] = sum_j ys[pad_pos[t,j]] + shared[t]
   moe::Range nvtx_combine("moe_permute_combine");
@@ -1686,8 +1684,8 @@ int lewi_moe_bwd(void* stream, void* side_stream, const void* dout, const void* 
   const bool shared = fs > 0;
   // the side stream takes the shared expert and, once dH has left the routing-weight gradient pieces, the router
   const bool fork = side_stream != nullptr && side_stream != stream;
-  moe::Events* ev = fork ? moe::events() : nullptr;
-  if (fork && ev == nullptr) return LEWI_ERR_CUDA;
+  const EventLease ev(fork);
+  if (fork && !ev.ok()) return LEWI_ERR_CUDA;
   void* sh_stream = fork ? side_stream : stream;
 
   const float* logits = reinterpret_cast<const float*>(res(LEWI_MOE_RES_LOGITS));
@@ -1705,8 +1703,7 @@ int lewi_moe_bwd(void* stream, void* side_stream, const void* dout, const void* 
 
   // shared expert backward: needs only dout, x and its own saved activations
   if (fork) {
-    if (cudaEventRecord(ev->fork_bwd, st) != cudaSuccess || cudaStreamWaitEvent(sd, ev->fork_bwd, 0) != cudaSuccess)
-      return LEWI_ERR_CUDA;
+    if (!stream_after(ev->fork, st, sd)) return LEWI_ERR_CUDA;
     moe::mark("side_begin", sh_stream);
   }
   auto shared_bwd = [&]() -> int {
@@ -1770,8 +1767,7 @@ int lewi_moe_bwd(void* stream, void* side_stream, const void* dout, const void* 
     return LEWI_OK;
   };
   if (fork) {
-    if (cudaEventRecord(ev->dh_done, st) != cudaSuccess || cudaStreamWaitEvent(sd, ev->dh_done, 0) != cudaSuccess)
-      return LEWI_ERR_CUDA;
+    if (!stream_after(ev->mid, st, sd)) return LEWI_ERR_CUDA;
     LEWI_TRY(router_bwd());
   }
   LEWI_TRY(lewi_grouped_gemm_tn(stream, res(LEWI_MOE_RES_H), Wk + W.dys, dw_down, nullptr, pad_offsets, D.Mpad, f, d, E,
@@ -1795,8 +1791,7 @@ int lewi_moe_bwd(void* stream, void* side_stream, const void* dout, const void* 
     if (shared) LEWI_TRY(shared_bwd());
   }
   if (fork) {
-    if (cudaEventRecord(ev->join_bwd, sd) != cudaSuccess || cudaStreamWaitEvent(st, ev->join_bwd, 0) != cudaSuccess)
-      return LEWI_ERR_CUDA;
+    if (!stream_after(ev->join, sd, st)) return LEWI_ERR_CUDA;
   }
   // dispatch backward: dx[t] = sum_j dxs[pad_pos[t,j]] + shared-expert and router terms
   LEWI_TRY(lewi_gather_reduce(stream, Wk + W.dxs, pad_pos, nullptr, dxsh, Wk + W.dx_r, dx, T, k, d, LEWI_BF16, LEWI_BF16,
