@@ -186,15 +186,17 @@ int lewi_gather_rows(void* stream, const void* x, const int32_t* idx, const floa
 int lewi_dispatch_rows(void* stream, const void* x, const int32_t* pos, const int32_t* row_slot, void* out,
                        int64_t T, int k, int d, int64_t out_rows, const int32_t* n_rows_dev, int rows_per_unit);
 
-/* The same without padding, `dispatch` of modal/moe_permute.py:270-289: out[pos[t,j]] = x[t], out [T*k,d] in dtype, pos a permutation
- * of the T*k rows.  k <= 32. */
-int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* pos, void* out, int64_t T, int k, int d, int dtype);
+/* The same without padding, `dispatch` of modal/moe_permute.py:270-289: out[r] = x[order[r] / k], out [T*k,d] in dtype, order i32 [T*k]
+ * the slot of every row (negative: a zero row), pos i32 [T,k] the row of every slot (negative: none).  Where the two are inverse
+ * permutations each source row is read once; rows for which they are not are written one by one.  order may be null: pos is then a
+ * permutation of the rows, a position that is no row is skipped and raises LEWI_STATUS_BAD_INDEX.  k <= 32. */
+int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* order, const int32_t* pos, void* out, int64_t T, int k, int d, int dtype);
 
-/* Both gradients of `combine` (modal/moe_permute.py:292-312) in one pass: dy[pos[t,j]] = w[t,j] * g[t] and dw[t,j] = <g[t], y[pos[t,j]]>
- * (f32), y, dy [n*k,d] in dtype, pos i32 [n,k] a permutation of the rows, w, dw f32 [n,k]; g [n,d] in dtype or f32, rounded to dtype
- * first.  k <= 32. */
-int lewi_combine_bwd(void* stream, const void* y, const int32_t* pos, const void* g, const float* w, void* dy, float* dw,
-                     int64_t n, int k, int d, int dtype, int g_dtype);
+/* Both gradients of `combine` (modal/moe_permute.py:292-312) in one pass: dy[r] = w_flat[order[r]] * g[order[r] / k] (zeros where order[r]
+ * is negative) and dw[t,j] = <g[t], y[pos[t,j]]> (f32; 0 where pos is negative), y [n_y_rows,d], dy [n_dy_rows,d] in dtype, order i32
+ * [n_dy_rows] (may be null, as above), pos i32 [n,k], w, dw f32 [n,k]; g [n,d] in dtype or f32, rounded to dtype first.  k <= 32. */
+int lewi_combine_bwd(void* stream, const void* y, const int32_t* order, const int32_t* pos, const void* g, const float* w, void* dy, float* dw,
+                     int64_t n, int k, int d, int64_t n_y_rows, int64_t n_dy_rows, int dtype, int g_dtype);
 
 /* out[t] = sum_j w[t,j] * y[pos[t,j]] (+ add0[t] + add1[t]) accumulated in f32.
  * w, add0, add1 may be null.  in_dtype: dtype of y/add0/add1; out_dtype: dtype of out.

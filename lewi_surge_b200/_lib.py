@@ -43,8 +43,8 @@ SIGNATURES = {
     "lewi_ragged_gemm_ok": (c_int, [c_int64, c_int]),
     "lewi_group_offsets": (c_int, [P, P, c_int, P]),
     "lewi_ragged_gemm": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int]),
-    "lewi_dispatch_tokens": (c_int, [P, P, P, P, c_int64, c_int, c_int, c_int]),
-    "lewi_combine_bwd": (c_int, [P, P, P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int]),
+    "lewi_dispatch_tokens": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int]),
+    "lewi_combine_bwd": (c_int, [P, P, P, P, P, P, P, P, c_int64, c_int, c_int, c_int64, c_int64, c_int, c_int]),
     "lewi_dispatch_rows": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int64, P, c_int]),
     "lewi_gather_reduce": (c_int, [P, P, P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int, c_int64]),
     "lewi_gather_dot": (c_int, [P, P, P, P, P, c_int64, c_int, c_int, c_int, c_int64]),

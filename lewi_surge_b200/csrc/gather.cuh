@@ -89,21 +89,20 @@ __global__ void __launch_bounds__(kGatherThreads) gather_rows_kernel(
 // (row_slot[r] < 0) become zero rows.  Every output row has exactly one writer, so this is the same function as
 // the row gather out[r] = x[row_slot[r] / k] -- but each source row is read once instead of k times at k distant
 // moments, which keeps the read side at T rows of DRAM traffic however large the source is against the L2.
-// (5003 tokens, k = 6, d = 1024, float32, no padding: 23 us, the row gather 35; 16,384 tokens, k = 12, d = 2048, bf16: 140 and 240.)
-// row_slot null: there are none.  A warp looks at ZR rows at a time for those to zero: 4 while no warp of the grid looks more than twice (kZeroRows), since at decode
+// A warp looks at ZR rows at a time for those to zero: 4 while no warp of the grid looks more than twice (kZeroRows), since at decode
 // sizes nearly all rows are such rows (8 tokens over 128 experts: 6.1 MB of zeros; 13 us with 32 rows per warp, 7 us with 4);
 // 32 beyond, where hardly any are (k = 6, d = 256: 16,384 tokens over 16 experts 9.3 us with 4 and 9.8 with 32, 49,152 34 and 32,
 // 65,536 over 128 48 and 45).
 constexpr int kZeroRows = 4;
-template <typename T, int VPL, int ZR>
+template <int VPL, int ZR>
 __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
-    const T* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
-    T* __restrict__ out, long long n_tokens, int k, int d, long long out_rows,
+    const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ pos, const int32_t* __restrict__ row_slot,
+    __nv_bfloat16* __restrict__ out, long long n_tokens, int k, int d, long long out_rows,
     const int32_t* __restrict__ n_rows_dev, int rows_per_unit) {
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int nvec = d / Elem<T>::kPerVec;
+  const int nvec = d / 8;
   long long rows = out_rows;
   if (n_rows_dev != nullptr) rows = min(rows, (long long)n_rows_dev[0] * rows_per_unit);
   for (long long t = warp0; t < n_tokens; t += n_warps) {
@@ -128,7 +127,6 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
       }
     }
   }
-  if (row_slot == nullptr) return;
   // zero rows of the padded layout
   for (long long r0 = warp0 * ZR; r0 < rows; r0 += n_warps * ZR) {
     const long long r = r0 + lane;
@@ -138,6 +136,68 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
       for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + rr * d) + vi, make_uint4(0, 0, 0, 0));
     }
   }
+}
+
+// Rows of the unpadded operators, table by table: row r of the sorted order belongs to slot order[r] (negative: to none), slot s sits at row
+// pos[s] (negative: nowhere).  The kernels below go through the tokens in order and write the rows that their slots sit at; the two tables
+// need not be inverse permutations of one another (a caller may drop slots), so a slot writes the row only if the row names it back, and
+// rows_left_over() then visits the rows that no slot has written: each row is written once, with what `order` says of it.
+// put(row, slot) writes row `row` for slot `slot` (negative: zeros); whole warp.  The slots write rows below n_slot_rows.
+template <class Put>
+__device__ __forceinline__ void rows_left_over(const int32_t* __restrict__ order, const int32_t* __restrict__ pos, long long n_rows,
+                                               long long n_slot_rows, long long n_slots, long long warp0, long long n_warps, int lane, Put put) {
+  for (long long r0 = warp0 * kWarp; r0 < n_rows; r0 += n_warps * kWarp) {
+    const long long r = r0 + lane;
+    const int s = r < n_rows ? order[r] : -1;
+    if (s >= n_slots) raise_status(LEWI_STATUS_BAD_INDEX);
+    const bool left = r < n_rows && s < n_slots && (s < 0 || r >= n_slot_rows || pos[s] != r);
+    for (unsigned m = __ballot_sync(0xffffffffu, left); m != 0; m &= m - 1) {
+      const int from = __ffs(m) - 1;
+      put(r0 + from, __shfl_sync(0xffffffffu, s, from));
+    }
+  }
+}
+// The row of this lane's slot, -1 where nothing is to be written for it.  Without `order` pos is a permutation: a slot without a row is an error.
+__device__ __forceinline__ int row_of_slot(const int32_t* __restrict__ order, int p, long long slot, long long n_rows) {
+  const bool in = p >= 0 && p < n_rows;
+  if (order == nullptr && !in) raise_status(LEWI_STATUS_BAD_INDEX);
+  return in && (order == nullptr || order[p] == slot) ? p : -1;
+}
+
+// out[r] = x[order[r] / k], in token order: every row of x is read once.
+template <typename T, int VPL>
+__global__ void __launch_bounds__(kGatherThreads) dispatch_tokens_kernel(const T* __restrict__ x, const int32_t* __restrict__ order,
+                                                                         const int32_t* __restrict__ pos, T* __restrict__ out,
+                                                                         long long n_tokens, int k, int d) {
+  const int lane = threadIdx.x & 31;
+  const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5, rows = n_tokens * k;
+  const int nvec = d / Elem<T>::kPerVec;
+  for (long long t = warp0; t < n_tokens; t += n_warps) {
+    const int my_row = lane < k ? row_of_slot(order, pos[t * k + lane], t * k + lane, rows) : -1;
+    uint4 v[VPL];
+#pragma unroll
+    for (int c = 0; c < VPL; ++c) {
+      const int vi = lane + c * kWarp;
+      v[c] = make_uint4(0, 0, 0, 0);
+      if (vi < nvec) v[c] = ld_nc_v4(reinterpret_cast<const uint4*>(x + t * d) + vi);
+    }
+    for (int j = 0; j < k; ++j) {
+      const long long p = __shfl_sync(0xffffffffu, my_row, j);
+      if (p < 0) continue;
+#pragma unroll
+      for (int c = 0; c < VPL; ++c) {
+        const int vi = lane + c * kWarp;
+        if (vi < nvec) st_v4(reinterpret_cast<uint4*>(out + p * d) + vi, v[c]);
+      }
+    }
+  }
+  if (order == nullptr) return;
+  rows_left_over(order, pos, rows, rows, rows, warp0, n_warps, lane, [&](long long r, int s) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)(s < 0 ? 0 : s / k) * d);
+#pragma unroll 1
+    for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + r * d) + vi, s < 0 ? make_uint4(0, 0, 0, 0) : ld_nc_v4(src + vi));
+  });
 }
 
 // out[t] = sum_j w[t,j] * y[pos[t,j]] (+ add0[t] + add1[t]); f32 accumulate.
@@ -357,60 +417,63 @@ inline int gather_grid(long long rows) {
   return (int)ctas;
 }
 
-// smallest supported VPL in {1,2,4,8,16} covering the row, or 0
-// Gradients of the combine, both in one pass over y, in token order: dy[pos[t,j]] = w[t,j] * g[t] and dw[t,j] = <g[t], y[pos[t,j]]>,
-// g in y's type (a float32 g is rounded here).  pos is a permutation, so every row of dy has one writer; a row of g is read once, not
-// k times, and a warp requests the next row of y while it works on one.
+// Gradients of the combine, both in one pass over y, in token order: dy[r] = w[order[r]] * g[order[r] / k] and dw[t,j] = <g[t], y[pos[t,j]]>,
+// g in y's type (a float32 g is rounded here).  Where the tables are inverse permutations a row of g is read once, not k times; a warp
+// requests the next row of y while it works on one.
 // 5003 tokens, k = 6, d = 1024, float32: 47 us (scaled gather and dots 35 + 39); 16,384 tokens, k = 12, d = 2048, bf16: 328 us, 5.3 TB/s
 // (240 + 207 and 32 for the rounded copy of g).  A warp per row of y instead, g out of L2 k times: 55 and 472 us.
 template <typename T, typename TG, int VPL>
-__global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __restrict__ y, const int32_t* __restrict__ pos,
-                                                                     const TG* __restrict__ g, const float* __restrict__ w,
-                                                                     T* __restrict__ dy, float* __restrict__ dw, long long n, int k, int d) {
+__global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __restrict__ y, const int32_t* __restrict__ order,
+                                                                     const int32_t* __restrict__ pos, const TG* __restrict__ g,
+                                                                     const float* __restrict__ w, T* __restrict__ dy, float* __restrict__ dw,
+                                                                     long long n, int k, int d, long long n_y_rows, long long n_dy_rows) {
   constexpr int PV = Elem<T>::kPerVec, GV = PV * sizeof(TG) / 16;   // vectors of g per vector of y
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5, m = n * k;
+  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int nvec = d / PV;
   const uint4 zero = make_uint4(0, 0, 0, 0);
+  const long long n_rows = min(n_y_rows, n_dy_rows);   // of these the slots take care
+  auto g_vec = [&](long long t, int vi) {   // a vector of g[t] in y's type
+    if constexpr (GV == 2) {   // float32 -> bf16
+      const uint4* src = reinterpret_cast<const uint4*>(g + t * d) + (long long)vi * 2;
+      const uint4 a = ld_nc_v4(src), b = ld_nc_v4(src + 1);
+      auto two = [](uint32_t lo, uint32_t hi) { return pack_bf16(__uint_as_float(lo), __uint_as_float(hi)); };
+      return make_uint4(two(a.x, a.y), two(a.z, a.w), two(b.x, b.y), two(b.z, b.w));
+    } else {
+      return ld_nc_v4(reinterpret_cast<const uint4*>(g + t * d) + vi);
+    }
+  };
   for (long long t = warp0; t < n; t += n_warps) {
     const int my_pos = lane < k ? pos[t * k + lane] : -1;
+    const int my_row = lane < k ? row_of_slot(order, my_pos, t * k + lane, n_rows) : -1;
+    if (my_pos >= n_y_rows) raise_status(LEWI_STATUS_BAD_INDEX);
     const float my_w = lane < k ? w[t * k + lane] : 0.f;
     uint4 gv[VPL], yv[VPL], next[VPL];
     auto fetch = [&](int j, uint4 (&v)[VPL]) {
-      const long long p = __shfl_sync(0xffffffffu, my_pos, j);
+      const long long p = __shfl_sync(0xffffffffu, my_row, j);
 #pragma unroll
       for (int c = 0; c < VPL; ++c) {
         const int vi = lane + c * kWarp;
-        v[c] = vi < nvec && p >= 0 && p < m ? ld_nc_v4(reinterpret_cast<const uint4*>(y + p * d) + vi) : zero;
+        v[c] = vi < nvec && p >= 0 ? ld_nc_v4(reinterpret_cast<const uint4*>(y + p * d) + vi) : zero;
       }
     };
     fetch(0, yv);
 #pragma unroll
     for (int c = 0; c < VPL; ++c) {
       const int vi = lane + c * kWarp;
-      if (vi >= nvec) gv[c] = zero;
-      else if constexpr (GV == 2) {   // float32 -> bf16
-        const uint4* src = reinterpret_cast<const uint4*>(g + t * d) + (long long)vi * 2;
-        const uint4 a = ld_nc_v4(src), b = ld_nc_v4(src + 1);
-        auto two = [](uint32_t lo, uint32_t hi) { return pack_bf16(__uint_as_float(lo), __uint_as_float(hi)); };
-        gv[c] = make_uint4(two(a.x, a.y), two(a.z, a.w), two(b.x, b.y), two(b.z, b.w));
-      } else {
-        gv[c] = ld_nc_v4(reinterpret_cast<const uint4*>(g + t * d) + vi);
-      }
+      gv[c] = vi < nvec ? g_vec(t, vi) : zero;
     }
     float my_dot = 0.f;
     for (int j = 0; j < k; ++j) {
       if (j + 1 < k) fetch(j + 1, next);
-      const long long p = __shfl_sync(0xffffffffu, my_pos, j);
+      const long long p = __shfl_sync(0xffffffffu, my_row, j);
       const float s = __shfl_sync(0xffffffffu, my_w, j);
-      const bool in = p >= 0 && p < m;
-      if (p >= m && lane == 0) raise_status(LEWI_STATUS_BAD_INDEX);
       float dot = 0.f;
 #pragma unroll
       for (int c = 0; c < VPL; ++c) {
         const int vi = lane + c * kWarp;
-        if (vi < nvec && in) {
+        if (vi < nvec && p >= 0) {
           float f[PV], q[PV];
           Elem<T>::unpack(yv[c], f);
           Elem<T>::unpack(gv[c], q);
@@ -426,8 +489,40 @@ __global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __
       dot = warp_sum(dot);
       if (lane == j) my_dot = dot;
     }
+    // slots at a row that is another slot's: only their dots
+    for (unsigned m = __ballot_sync(0xffffffffu, my_row < 0 && my_pos >= 0 && my_pos < n_y_rows); m != 0; m &= m - 1) {
+      const int j = __ffs(m) - 1;
+      const long long p = __shfl_sync(0xffffffffu, my_pos, j);
+      float dot = 0.f;
+#pragma unroll 1
+      for (int vi = lane; vi < nvec; vi += kWarp) {
+        float f[PV], q[PV];
+        Elem<T>::unpack(ld_nc_v4(reinterpret_cast<const uint4*>(y + p * d) + vi), f);
+        Elem<T>::unpack(g_vec(t, vi), q);
+#pragma unroll
+        for (int e = 0; e < PV; ++e) dot = fmaf(q[e], f[e], dot);
+      }
+      dot = warp_sum(dot);
+      if (lane == j) my_dot = dot;
+    }
     if (lane < k) dw[t * k + lane] = my_dot;
   }
+  if (order == nullptr) return;
+  rows_left_over(order, pos, n_dy_rows, n_rows, n * k, warp0, n_warps, lane, [&](long long r, int s) {
+    const float sc = s < 0 ? 0.f : w[s];
+#pragma unroll 1
+    for (int vi = lane; vi < nvec; vi += kWarp) {
+      uint4 v = zero;
+      if (s >= 0) {
+        float q[PV];
+        Elem<T>::unpack(g_vec(s / k, vi), q);
+#pragma unroll
+        for (int e = 0; e < PV; ++e) q[e] *= sc;
+        v = Elem<T>::pack(q);
+      }
+      st_v4(reinterpret_cast<uint4*>(dy + r * d) + vi, v);
+    }
+  });
 }
 
 // Padded rows of the experts that have more than one row block: row r = x[row_slot[r] / k], zeros where row_slot[r] < 0; other experts'
@@ -455,6 +550,7 @@ __global__ void __launch_bounds__(256) gather_heavy_kernel(const __nv_bfloat16* 
   }
 }
 
+// smallest supported VPL in {1,2,4,8,16} covering the row, or 0
 inline int pick_vpl(int d, int elem_bytes) {
   const long long row_bytes = (long long)d * elem_bytes;
   if (row_bytes % 16 != 0) return 0;

@@ -33,7 +33,7 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 extern "C" {
 
-int lewi_version(void) { return 100; }
+int lewi_version(void) { return 101; }
 
 const char* lewi_error_string(int code) {
   switch (code) {
@@ -257,7 +257,7 @@ int lewi_dispatch_rows(void* stream, const void* x, const int32_t* pos, const in
   cudaStream_t st = as_stream(stream);
   const long long looks = out_rows / kZeroRows + 1;   // of warps at kZeroRows rows each
 #define LEWI_DR(ZR)                                                                                                   \
-  LEWI_DISPATCH_VPL(vpl, (dispatch_rows_kernel<__nv_bfloat16, VPL, ZR><<<gather_grid(T > out_rows / ZR ? T : out_rows / ZR + 1),      \
+  LEWI_DISPATCH_VPL(vpl, (dispatch_rows_kernel<VPL, ZR><<<gather_grid(T > out_rows / ZR ? T : out_rows / ZR + 1),      \
                                                           kGatherThreads, 0, st>>>(                                   \
                              reinterpret_cast<const __nv_bfloat16*>(x), pos, row_slot,                                \
                              reinterpret_cast<__nv_bfloat16*>(out), T, k, d, out_rows, n_rows_dev, rows_per_unit)))
@@ -268,7 +268,7 @@ int lewi_dispatch_rows(void* stream, const void* x, const int32_t* pos, const in
   return LEWI_OK;
 }
 
-int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* pos, void* out, int64_t T, int k, int d, int dtype) {
+int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* order, const int32_t* pos, void* out, int64_t T, int k, int d, int dtype) {
   if (!x || !pos || !out || T < 0 || k <= 0 || d <= 0 || (dtype != LEWI_BF16 && dtype != LEWI_F32)) return LEWI_ERR_ARG;
   if (k > kWarp) return LEWI_ERR_LIMIT;
   if (!aligned16(x) || !aligned16(out)) return LEWI_ERR_SHAPE;
@@ -278,8 +278,8 @@ int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* pos, void* 
   cudaStream_t st = as_stream(stream);
   const int grid = gather_grid(T);
 #define LEWI_DT(TT)                                                                                                     \
-  LEWI_DISPATCH_VPL(vpl, (dispatch_rows_kernel<TT, VPL, kWarp><<<grid, kGatherThreads, 0, st>>>(                          \
-                             reinterpret_cast<const TT*>(x), pos, nullptr, reinterpret_cast<TT*>(out), T, k, d, T * k, nullptr, 1)))
+  LEWI_DISPATCH_VPL(vpl, (dispatch_tokens_kernel<TT, VPL><<<grid, kGatherThreads, 0, st>>>(                               \
+                             reinterpret_cast<const TT*>(x), order, pos, reinterpret_cast<TT*>(out), T, k, d)))
   if (dtype == LEWI_BF16) { LEWI_DT(__nv_bfloat16); }
   else { LEWI_DT(float); }
 #undef LEWI_DT
@@ -287,20 +287,21 @@ int lewi_dispatch_tokens(void* stream, const void* x, const int32_t* pos, void* 
   return LEWI_OK;
 }
 
-int lewi_combine_bwd(void* stream, const void* y, const int32_t* pos, const void* g, const float* w, void* dy, float* dw, int64_t n, int k,
-                     int d, int dtype, int g_dtype) {
-  if (!y || !pos || !g || !w || !dy || !dw || n < 0 || k <= 0 || d <= 0) return LEWI_ERR_ARG;
+int lewi_combine_bwd(void* stream, const void* y, const int32_t* order, const int32_t* pos, const void* g, const float* w, void* dy, float* dw,
+                     int64_t n, int k, int d, int64_t n_y_rows, int64_t n_dy_rows, int dtype, int g_dtype) {
+  if (!y || !pos || !g || !w || !dy || !dw || n < 0 || k <= 0 || d <= 0 || n_y_rows < 0 || n_dy_rows < 0) return LEWI_ERR_ARG;
   if ((dtype != LEWI_BF16 && dtype != LEWI_F32) || (g_dtype != dtype && g_dtype != LEWI_F32)) return LEWI_ERR_ARG;
   if (k > kWarp) return LEWI_ERR_LIMIT;
   if (!aligned16(y) || !aligned16(g) || !aligned16(dy)) return LEWI_ERR_SHAPE;
   const int vpl = pick_vpl(d, dtype == LEWI_BF16 ? 2 : 4);
   if (vpl == 0) return LEWI_ERR_SHAPE;
-  if (n == 0) return LEWI_OK;
+  if (n == 0 && n_dy_rows == 0) return LEWI_OK;
   cudaStream_t st = as_stream(stream);
   const int grid = gather_grid(n);
 #define LEWI_CB(TT, TG)                                                                                                 \
   LEWI_DISPATCH_VPL(vpl, (combine_bwd_kernel<TT, TG, VPL><<<grid, kGatherThreads, 0, st>>>(                               \
-                             reinterpret_cast<const TT*>(y), pos, reinterpret_cast<const TG*>(g), w, reinterpret_cast<TT*>(dy), dw, n, k, d)))
+                             reinterpret_cast<const TT*>(y), order, pos, reinterpret_cast<const TG*>(g), w, reinterpret_cast<TT*>(dy), dw, n, k, d, \
+                             n_y_rows, n_dy_rows)))
   if (dtype == LEWI_F32) { LEWI_CB(float, float); }
   else if (g_dtype == LEWI_F32) { LEWI_CB(__nv_bfloat16, float); }
   else { LEWI_CB(__nv_bfloat16, __nv_bfloat16); }

@@ -132,29 +132,33 @@ def gather_dot(y, pos, g):
   return out
 
 
-def dispatch_tokens(x, pos, k):
-  """out[pos[t*k+j]] = x[t] for a permutation pos of the N*k rows: equals ``gather_rows(x, order, idx_div=k)`` for its inverse, reading
-  every row once."""
+def dispatch_tokens(x, pos, k, order=None):
+  """``gather_rows(x, order, idx_div=k)``, reading every row once where pos (N*k) is the inverse of order; without order pos is a
+  permutation of the N*k rows and out[pos[t*k+j]] = x[t]."""
   lib = _lib.load()
   x, pos = x.contiguous(), _i32(pos).contiguous()
+  order = None if order is None else _i32(order).contiguous()
   t, d = x.shape
   out = torch.empty((t * k, d), dtype=x.dtype, device=x.device)
-  check(lib.lewi_dispatch_tokens(stream(), ptr(x), ptr(pos), ptr(out), t, k, d, _dt(x)), "lewi_dispatch_tokens")
+  check(lib.lewi_dispatch_tokens(stream(), ptr(x), ptr(order), ptr(pos), ptr(out), t, k, d, _dt(x)), "lewi_dispatch_tokens")
   return out
 
 
-def combine_bwd(y, pos, g, w):
-  """(dy, dw f32) of ``combine`` for a permutation pos (N, k): dy[pos[t,j]] = w[t,j] * g[t], dw[t,j] = <g[t], y[pos[t,j]]>, g rounded to
-  y.dtype."""
+def combine_bwd(y, pos, g, w, order=None):
+  """(dy, dw f32) of ``combine``: dy[r] = w_flat[order[r]] * g[order[r] // k], zeros where order[r] < 0, and dw[t,j] = <g[t], y[pos[t,j]]>, 0
+  where pos[t,j] < 0; g rounded to y.dtype.  Without order pos is a permutation of the N*k rows and order its inverse."""
   lib = _lib.load()
   y, pos, w = y.contiguous(), _i32(pos).contiguous(), w.to(torch.float32).contiguous()
   g = (g if g.dtype in (y.dtype, torch.float32) else g.to(y.dtype)).contiguous()
   (n, k), d = w.shape, y.shape[1]
-  if y.shape[0] != n * k or pos.numel() != n * k or g.shape != (n, d):
+  order = None if order is None else _i32(order).contiguous()
+  if pos.numel() != n * k or g.shape != (n, d) or (order is None and y.shape[0] != n * k):
     raise LewiError("combine_bwd: y (N*k, D), pos (N, k), g (N, D), w (N, k)")
-  dy, dw = torch.empty_like(y), torch.empty_like(w)
+  rows = n * k if order is None else order.shape[0]
+  dy, dw = torch.empty((rows, d), dtype=y.dtype, device=y.device), torch.empty_like(w)
   if n * k > 0:
-    check(lib.lewi_combine_bwd(stream(), ptr(y), ptr(pos), ptr(g), ptr(w), ptr(dy), ptr(dw), n, k, d, _dt(y), _dt(g)), "lewi_combine_bwd")
+    check(lib.lewi_combine_bwd(stream(), ptr(y), ptr(order), ptr(pos), ptr(g), ptr(w), ptr(dy), ptr(dw), n, k, d, y.shape[0], rows, _dt(y),
+                               _dt(g)), "lewi_combine_bwd")
   return dy, dw
 
 
@@ -194,7 +198,7 @@ class _Dispatch(torch.autograd.Function):
     ctx.save_for_backward(pos)
     ctx.n, ctx.k, ctx.dtype = n, k, x.dtype
     if 0 < k <= 32 and k * n == order.shape[0] == pos.shape[0]:
-      return dispatch_tokens(x, pos, k)
+      return dispatch_tokens(x, pos, k, order)
     return gather_rows(x, order, idx_div=k)
 
   @staticmethod
@@ -209,13 +213,13 @@ class _Combine(torch.autograd.Function):
   @staticmethod
   def forward(ctx, y, order, pos, w):
     n, k = w.shape
-    ctx.save_for_backward(y, pos, w)
+    ctx.save_for_backward(y, order, pos, w)
     return gather_reduce(y, pos.view(n, k), w, torch.float32)
 
   @staticmethod
   def backward(ctx, g):
-    y, pos, w = ctx.saved_tensors
-    dy, dw = combine_bwd(y, pos, g, w)
+    y, order, pos, w = ctx.saved_tensors
+    dy, dw = combine_bwd(y, pos, g, w, order)
     return dy, None, None, dw.to(w.dtype)
 
 
@@ -236,12 +240,14 @@ class _PermuteRows(torch.autograd.Function):
 
 
 def dispatch(x, order, pos):
-  """Reference: dispatch, modal/moe_permute.py:270-289."""
+  """Row p is x[order[p] // k], a zero row where order[p] < 0; pos (N*k) is the row of every slot, negative for one that has none.
+  Reference: dispatch, modal/moe_permute.py:270-289."""
   return _Dispatch.apply(x, _i32(order), _i32(pos))
 
 
 def combine(y, order, pos, w):
-  """Reference: combine, modal/moe_permute.py:292-312."""
+  """sum_j w[t,j] * y[pos[t,j]] in float32, a negative pos adds nothing; order names the slot of every row for y's gradient (negative: none).
+  Reference: combine, modal/moe_permute.py:292-312."""
   return _Combine.apply(y, _i32(order), _i32(pos), w)
 
 

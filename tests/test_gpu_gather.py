@@ -182,3 +182,62 @@ def test_token_order_dispatch_and_combine_gradients_equal_the_row_gathers(cuda, 
   got = torch.autograd.grad(ops.combine(y, order, pos, w), (y, w), g.float())
   assert torch.equal(got[0], dy) and torch.equal(got[1], dw)
   assert _lib.last_status() == 0
+
+
+@pytest.mark.parametrize("t,k,d,dtype", [(1, 2, 8, "bf16"), (50, 6, 264, "f32"), (700, 4, 1024, "bf16"), (40, 12, 2048, "f32"), (6000, 3, 64, "bf16")])
+@pytest.mark.parametrize("tables", ["dropped", "order_only", "pos_only", "unrelated", "short"])
+def test_dispatch_and_combine_with_tables_that_are_no_permutations(cuda, t, k, d, dtype, tables):
+  """Slots that were dropped (both tables negative, or one of them), tables that do not belong together, rows left out of order: every row is
+  what the row gathers make of `order`, every sum and dot what `pos` names, and nothing is left unwritten."""
+  from lewi_surge_b200 import ops, _lib
+  dt = dict(bf16=torch.bfloat16, f32=torch.float32)[dtype]
+  gen = torch.Generator(device=cuda).manual_seed(t + k)
+  rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda)
+  m = t * k
+  order = torch.randperm(m, generator=gen, device=cuda).to(torch.int32)
+  pos = torch.empty_like(order)
+  pos[order.long()] = torch.arange(m, dtype=torch.int32, device=cuda)
+  gone = torch.rand(m, generator=gen, device=cuda) < 0.3
+  gone[0] = True
+  rows = m
+  if tables in ("dropped", "pos_only"):
+    pos[order[gone].long()] = -1
+  if tables in ("dropped", "order_only"):
+    order[gone] = -1
+  if tables == "unrelated":   # some rows name the same slot, some slots the same row, out of range of nothing
+    order = torch.randint(-1, m, (m,), generator=gen, device=cuda, dtype=torch.int32)
+    pos = torch.randint(-1, m, (m,), generator=gen, device=cuda, dtype=torch.int32)
+  if tables == "short":       # the dropped slots' rows do not exist at all
+    rows = m // 2 + 1
+    order = order[:rows].contiguous()
+    pos = torch.where(pos < rows, pos, -1)
+  x, y, w, g = rnd(t, d).to(dt), rnd(rows, d).to(dt), rnd(t, k), rnd(t, d)
+  junk = torch.full((4 * m * d,), float("nan"), device=cuda)
+  del junk                    # what a fresh output may hold
+  _lib.last_status()
+  x.requires_grad_(True)
+  if tables != "short":       # (k of the dispatch follows from the rows)
+    out = ops.dispatch(x, order, pos)
+    assert torch.equal(out, ops.gather_rows(x, order, idx_div=k))
+    dx, = torch.autograd.grad(out, x, y)
+    assert torch.equal(dx, ops.gather_reduce(y, pos.view(t, k), None, dt))
+  y.requires_grad_(True)
+  w.requires_grad_(True)
+  dy, dw = torch.autograd.grad(ops.combine(y, order, pos, w), (y, w), g)
+  gy = g.to(dt)
+  assert torch.equal(dy, ops.gather_rows(gy, order, w.detach().reshape(-1), idx_div=k, scale_by_idx=True))
+  assert torch.equal(dw, ops.gather_dot(y.detach(), pos.view(t, k), gy))
+  assert _lib.last_status() == 0
+
+
+def test_a_slot_without_a_row_is_an_error_where_pos_alone_is_given(cuda):
+  from lewi_surge_b200 import ops, _lib
+  x, pos = torch.randn(2, 64, device=cuda), torch.tensor([0, 3, -1, 1], dtype=torch.int32, device=cuda)
+  _lib.last_status()
+  ops.dispatch_tokens(x, pos, 2)
+  assert _lib.last_status() & _lib.STATUS_BAD_INDEX
+  ops.combine_bwd(torch.randn(4, 64, device=cuda), pos.view(2, 2), x, torch.rand(2, 2, device=cuda))
+  assert _lib.last_status() & _lib.STATUS_BAD_INDEX
+  order = torch.tensor([0, 3, 4, 1], dtype=torch.int32, device=cuda)   # slot 4 of four: skipped and reported, as by gather_rows
+  ops.dispatch(x, order, pos)
+  assert _lib.last_status() & _lib.STATUS_BAD_INDEX
