@@ -149,7 +149,9 @@ def combine_bwd(y, pos, g, w, order=None):
   where pos[t,j] < 0; g rounded to y.dtype.  Without order pos is a permutation of the N*k rows and order its inverse."""
   lib = _lib.load()
   y, pos, w = y.contiguous(), _i32(pos).contiguous(), w.to(torch.float32).contiguous()
-  g = (g if g.dtype in (y.dtype, torch.float32) else g.to(y.dtype)).contiguous()
+  g = g.contiguous()
+  if g.dtype != y.dtype and (g.dtype != torch.float32 or g.data_ptr() % 16):   # (the kernel rounds float32 rows that start on 16 bytes)
+    g = g.to(y.dtype)
   (n, k), d = w.shape, y.shape[1]
   order = None if order is None else _i32(order).contiguous()
   if pos.numel() != n * k or g.shape != (n, d) or (order is None and y.shape[0] != n * k):
