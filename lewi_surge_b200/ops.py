@@ -347,7 +347,8 @@ def _ragged_gemm(a, b, offsets, transposed):
 class _RaggedDot(torch.autograd.Function):
   """Dropless grouped GEMM.  The products over rows run on the rows as they come (gathered into padded groups and back they took two
   passes over them each: 36,006 rows over 64 groups, 1024 x 512, forward 82 -> 51 us); the weight gradient contracts over rows and reads
-  them gathered into padded groups.
+  them gathered into padded groups.  lhs is gathered in the forward pass, and only where a gradient of rhs will be asked for: what is saved
+  is not the caller's lhs, which may change before the backward pass.
 
   Reference: padded_ragged_dot, modal/padded_gmm.py:45-69 (and te_ragged_dot, modal/te_gmm.py:12-19
   for the dropless semantics): rows of lhs are sorted by expert, group g multiplies rhs[g], rows past
@@ -355,7 +356,7 @@ class _RaggedDot(torch.autograd.Function):
   """
 
   @staticmethod
-  def forward(ctx, lhs, rhs, group_sizes):
+  def forward(ctx, lhs, rhs, group_sizes, rhs_grad):
     lib = _lib.load()
     m, k = lhs.shape
     e, n = rhs.shape[0], rhs.shape[2]
@@ -367,7 +368,11 @@ class _RaggedDot(torch.autograd.Function):
       gs = _i32(group_sizes).contiguous()
       offsets = torch.empty(e + 1, dtype=torch.int32, device=gs.device)
       check(lib.lewi_group_offsets(stream(), ptr(gs), e, ptr(offsets)), "lewi_group_offsets")
-      ctx.save_for_backward(a, b, offsets)   # (not the sizes, which the caller may overwrite for the next call)
+      rows = ()
+      if rhs_grad:
+        t = group_tables(gs, m)
+        rows = (gather_rows(a, t["row_of_padded"]), t["row_of_padded"], t["pad_offsets"])
+      ctx.save_for_backward(b, offsets, *rows)   # (not the sizes, which the caller may overwrite for the next call)
       return _ragged_gemm(a, b, offsets, False).to(lhs.dtype)
     t = group_tables(group_sizes, m)
     buf = gather_rows(a, t["row_of_padded"])
@@ -381,17 +386,19 @@ class _RaggedDot(torch.autograd.Function):
   def backward(ctx, g):
     g = g.to(torch.bfloat16).contiguous()
     if ctx.compact:
-      a, b, offsets = ctx.saved_tensors
+      b, offsets, *rows = ctx.saved_tensors
       dlhs = _ragged_gemm(g, b, offsets, True)   # g . rhs[e]^T: rhs [E,K,N] read as the K-major operand with contraction over N
-      t = group_tables(offsets[1:] - offsets[:-1], a.shape[0])
-      buf, g_pad, pad_offsets = gather_rows(a, t["row_of_padded"]), gather_rows(g, t["row_of_padded"]), t["pad_offsets"]
+      if not rows:
+        return dlhs.to(ctx.lhs_dtype), None, None, None
+      buf, row_of_padded, pad_offsets = rows
+      g_pad = gather_rows(g, row_of_padded)
     else:
       buf, b, row_of_padded, padded_of_row, block_expert, n_blocks, pad_offsets = ctx.saved_tensors
       g_pad = gather_rows(g, row_of_padded)
       dlhs = gather_rows(grouped_gemm_nt(g_pad, b, block_expert, n_blocks, pad_offsets=pad_offsets), padded_of_row)
     # rounded once from the float32 accumulators where the weights are bf16
     drhs = grouped_gemm_tn(buf, g_pad, pad_offsets, ctx.e, out_dtype=torch.bfloat16 if ctx.rhs_dtype == torch.bfloat16 else torch.float32)
-    return dlhs.to(ctx.lhs_dtype), drhs.to(ctx.rhs_dtype), None
+    return dlhs.to(ctx.lhs_dtype), drhs.to(ctx.rhs_dtype), None, None
 
 
 def ragged_dot(lhs, rhs, group_sizes, precision=None, preferred_element_type=None, **kw):
@@ -399,7 +406,7 @@ def ragged_dot(lhs, rhs, group_sizes, precision=None, preferred_element_type=Non
   del precision, preferred_element_type
   if lhs.dim() != 2 or rhs.dim() != 3 or kw.get("group_offset") is not None:
     raise LewiError("ragged_dot: only lhs [M,K], rhs [E,K,N] without group_offset is supported")
-  return _RaggedDot.apply(lhs, rhs, _i32(group_sizes))
+  return _RaggedDot.apply(lhs, rhs, _i32(group_sizes), torch.is_grad_enabled() and rhs.requires_grad)
 
 
 padded_ragged_dot = ragged_dot

@@ -419,3 +419,23 @@ def test_ragged_product_with_offsets_gone_wrong_stays_within_its_output(cuda, of
   if list(offsets) == sorted(offsets) and offsets[:2] == (0, 40):
     want = a[:40].float() @ (b[0].float().T if transposed else b[0].float())
     assert O.rel_err(to_np(out[:40].float()), to_np(want)) <= TOL
+
+
+@pytest.mark.parametrize("lhs_grad,rhs_grad", [(True, True), (False, True), (True, False)])
+def test_ragged_dot_gradients_do_not_depend_on_lhs_staying_as_it_was(cuda, lhs_grad, rhs_grad):
+  """lhs may be overwritten between the passes (an activation buffer that is used again); gradients that are not asked for are left out."""
+  from lewi_surge_b200 import ops
+  gen = torch.Generator(device=cuda).manual_seed(3)
+  sizes = torch.tensor([70, 0, 131, 9], dtype=torch.int32, device=cuda)
+  base, rhs, g = (torch.randn(*s, generator=gen, device=cuda).bfloat16() for s in ((215, 64), (4, 64, 72), (215, 72)))
+  def grads(overwrite):
+    leaf, b = base.clone().requires_grad_(lhs_grad), rhs.clone().requires_grad_(rhs_grad)
+    a = leaf * 1
+    out = ops.ragged_dot(a, b, sizes)
+    if overwrite:
+      with torch.no_grad():
+        a.zero_()
+    return torch.autograd.grad(out, [t for t in (leaf, b) if t.requires_grad], g)
+  for x, y in zip(grads(True), grads(False)):
+    assert x.any() and torch.equal(x, y)
+  assert not ops.ragged_dot(base, rhs, sizes).requires_grad
