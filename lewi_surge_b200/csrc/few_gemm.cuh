@@ -71,10 +71,16 @@ struct Tile {
   int e, row0, valid, rows16, n0;   // rows16: valid rounded up to 16; 0: nothing to do
 };
 
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Barriers of the four epilogue warps.  bar.* wants each warp converged, which is not left to how the compiler joins the lanes of a wait
+// that they leave at different turns, or of a branch.
+__device__ __forceinline__ void epi_sync() {
+  __syncwarp();
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+}
 // the same barrier; whether p holds in one of the threads
 __device__ __forceinline__ bool epi_any(bool p) {
   uint32_t r;
+  __syncwarp();
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
                : "=r"(r) : "r"((uint32_t)p) : "memory");
   return r != 0;
@@ -287,7 +293,8 @@ few_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant_
       if (t.rows16 == 0) continue;
       const uint32_t acc = acc_it & 1u;
       // the four warps go on or leave together: one that left alone would keep the others at the barriers below
-      if (epi_any(!ptx::mbar_wait(tfull_bar(acc), (acc_it >> 1) & 1u, abort_flag))) break;
+      const bool got = ptx::mbar_wait(tfull_bar(acc), (acc_it >> 1) & 1u, abort_flag);
+      if (epi_any(!got)) break;
       ptx::tc_fence_after();
       for (int c = 0; c < t.rows16; c += 32) {
         uint32_t v[32];
