@@ -64,3 +64,64 @@ def test_router_logits_of_few_tokens(cuda, t, d, e):
   want = x.double() @ w.double() + b.double()
   got = layer.router_logits(x, w, b)
   assert float((got.double() - want).abs().max() / want.abs().max()) <= 1e-5
+
+
+def decode_weights(cuda, gen, d, e, f, fs):
+  from lewi_surge_b200 import layer
+  rnd = lambda *s: torch.randn(*s, generator=gen, device=cuda).bfloat16()
+  shared = (rnd(d, fs) * 0.02, rnd(d, fs) * 0.02, rnd(fs, d) * 0.02) if fs else (None, None, None)
+  return rnd, layer.MoEWeights(rnd(d, e).float() * 0.1, rnd(e, d, f) * 0.02, rnd(e, d, f) * 0.02, rnd(e, f, d) * 0.02, *shared)
+
+
+@pytest.mark.parametrize("t,d,e,f,fs,k", [(1, 256, 64, 128, 0, 2), (8, 1024, 128, 512, 512, 6), (64, 512, 256, 256, 0, 8), (512, 256, 64, 128, 192, 4)])
+def test_kernels_that_start_early_give_the_bits_of_those_that_wait(cuda, t, d, e, f, fs, k):
+  """Up to 512 tokens each kernel from the router on starts while the one before it ends, and the down projection reads the routing tables
+  before it waits; a mark callback keeps the launches apart.  Several steps in a row over other tokens, queued without a pause, in the same
+  buffers: tables or rows of the step before must not show."""
+  from lewi_surge_b200 import layer
+  gen = torch.Generator(device=cuda).manual_seed(t)
+  rnd, w = decode_weights(cuda, gen, d, e, f, fs)
+  xs = [rnd(t, d) for _ in range(6)]
+  def steps():
+    res = []
+    for x in xs * 3:
+      out, cache = layer.moe_layer_fwd(x, w, k)
+      rows = cache.tables.row_slot
+      h = cache.item("h", torch.bfloat16, (cache.tables.mpad, f))
+      res.append((out, cache.logits.clone(), cache.tables.topk_idx.clone(), rows.clone(), torch.where((rows >= 0)[:, None], h, 0)))
+      del out, cache, rows, h   # the next step's residual may take the same memory
+    return res
+  try:
+    layer.set_profile_hook(lambda *a: None)
+    apart = steps()
+  finally:
+    layer.set_profile_hook(None)
+  early = steps()
+  for u, v in zip(early, apart):
+    for p, q in zip(u, v):
+      assert torch.equal(p, q)
+  assert not torch.equal(early[0][2], early[1][2])
+
+
+@pytest.mark.parametrize("t,d,e,f,fs,k", [(1, 256, 64, 128, 0, 2), (8, 1024, 128, 512, 512, 6), (64, 512, 256, 256, 320, 8), (512, 256, 64, 128, 0, 4)])
+def test_captured_step_of_few_tokens_follows_its_inputs(cuda, t, d, e, f, fs, k):
+  """A decode step in a graph, replayed over changing tokens without a pause: the eager step's bits each time."""
+  from lewi_surge_b200 import layer
+  gen = torch.Generator(device=cuda).manual_seed(t)
+  rnd, w = decode_weights(cuda, gen, d, e, f, fs)
+  xs = [rnd(t, d) for _ in range(5)]
+  x = xs[0].clone()
+  def step():
+    out, cache = layer.moe_layer_fwd(x, w, k)
+    return out, cache.tables.topk_idx, cache.tables.counts
+  step()
+  captured = layer.CapturedStep(step)
+  got = []
+  for v in xs * 4:
+    x.copy_(v)
+    got.append([r.clone() for r in captured()])
+  for i, v in enumerate(xs * 4):
+    x.copy_(v)
+    for p, q in zip(got[i], step()):
+      assert torch.equal(p, q)
+  assert not torch.equal(got[0][1], got[1][1])
