@@ -406,6 +406,8 @@ def ragged_dot(lhs, rhs, group_sizes, precision=None, preferred_element_type=Non
   del precision, preferred_element_type
   if lhs.dim() != 2 or rhs.dim() != 3 or kw.get("group_offset") is not None:
     raise LewiError("ragged_dot: only lhs [M,K], rhs [E,K,N] without group_offset is supported")
+  if lhs.shape[1] != rhs.shape[1] or group_sizes.dim() != 1 or group_sizes.shape[0] < rhs.shape[0]:   # (the kernels would read past them)
+    raise LewiError(f"ragged_dot: lhs {tuple(lhs.shape)}, rhs {tuple(rhs.shape)} and group_sizes {tuple(group_sizes.shape)} do not fit")
   return _RaggedDot.apply(lhs, rhs, _i32(group_sizes), torch.is_grad_enabled() and rhs.requires_grad)
 
 

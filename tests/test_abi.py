@@ -130,3 +130,15 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
   monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "absent.so"))
   with pytest.raises(_lib.LewiError):
     _lib.load()
+
+
+def test_ragged_dot_refuses_sizes_that_do_not_fit():
+  """Before anything is launched: the kernels take the number of groups from rhs and the contraction from lhs, and would read past a shorter
+  table or weight."""
+  import torch
+  from lewi_surge_b200 import _lib, ops
+  lhs, rhs = torch.zeros(40, 64, dtype=torch.bfloat16), torch.zeros(8, 64, 48, dtype=torch.bfloat16)
+  for a, b, gs in ((lhs, rhs, torch.zeros(7, dtype=torch.int32)), (torch.zeros(40, 72, dtype=torch.bfloat16), rhs, torch.zeros(8, dtype=torch.int32)),
+                   (lhs, rhs, torch.zeros(8, 1, dtype=torch.int32))):
+    with pytest.raises(_lib.LewiError, match="do not fit"):
+      ops.ragged_dot(a, b, gs)
