@@ -180,7 +180,7 @@ struct Tile {
 // Rows [lo, hi) of the tensor that a group of the pair kernels (NN / NT) has by its offsets.  Offsets that lie outside the tensor or fall (a
 // table gone wrong) name no rows beyond it: every row that is stored lies in [0, rows).
 __device__ __forceinline__ int2 rows_of_group(const Args& a, int lo, int hi) {
-  const int n = (int)min(a.rows, 0x7fffffffLL);
+  const int n = (int)a.rows;   // (tensor maps take 32-bit rows)
   const int first = min(max(lo, 0), n);
   return make_int2(first, min(max(hi, first), n));
 }
@@ -265,11 +265,11 @@ __device__ __forceinline__ Tile decode_tile(const Args& a, int tile, int n_tiles
         }
         t.e = lo;
         const int2 r = rows_of_group(a, a.pad_offsets[lo], a.pad_offsets[lo + 1]);
-        const long long first = r.x + (unit - (long long)pp[lo]) * 2 * BM;
-        const bool in = first >= r.x && first < r.y;   // (else the groups overlap and have more pairs than 16 bits count: nothing is stored)
-        t.row0 = in ? (int)first : r.x;
+        const unsigned at = (unsigned)((unit - (int)pp[lo]) * 2 * BM), n = (unsigned)(r.y - r.x);
+        const bool in = at < n;   // (else the groups overlap and have more pairs than 16 bits count: nothing is stored)
+        t.row0 = in ? r.x + (int)at : r.x;
         t.row_end = in ? r.y : r.x;
-        t.second = (long long)t.row0 + BM < t.row_end;
+        t.second = in && at + BM < n;
       } else {
         t.e = 0;
         t.row0 = unit * 2 * BM;
