@@ -141,20 +141,20 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_rows_kernel(
 // Rows of the unpadded operators, table by table: row r of the sorted order belongs to slot order[r] (negative: to none), slot s sits at row
 // pos[s] (negative: nowhere).  The kernels below go through the tokens in order and write the rows that their slots sit at; the two tables
 // need not be inverse permutations of one another (a caller may drop slots), so a slot writes the row only if the row names it back, and
-// rows_left_over() then visits the rows that no slot has written: each row is written once, with what `order` says of it.
-// put(row, slot) writes row `row` for slot `slot` (negative: zeros); whole warp.  The slots write rows below n_slot_rows.
+// the rows left over, which no slot writes, are visited apart: each row is written once, with what `order` says of it.
+__device__ __forceinline__ int slot_of_row(const int32_t* __restrict__ order, long long r, long long n_rows) { return r < n_rows ? order[r] : -1; }
+// Which of a warp's 32 rows are left over, lane's row being r of slot s; the slots write rows below n_slot_rows.
+__device__ __forceinline__ unsigned left_over(const int32_t* __restrict__ pos, int s, long long r, long long n_rows, long long n_slot_rows,
+                                              long long n_slots) {
+  if (s >= n_slots) raise_status(LEWI_STATUS_BAD_INDEX);
+  return __ballot_sync(0xffffffffu, r < n_rows && s < n_slots && (s < 0 || r >= n_slot_rows || pos[s] != r));
+}
+// put(row, slot) writes row `row` for slot `slot` (negative: zeros); whole warp.
 template <class Put>
-__device__ __forceinline__ void rows_left_over(const int32_t* __restrict__ order, const int32_t* __restrict__ pos, long long n_rows,
-                                               long long n_slot_rows, long long n_slots, long long warp0, long long n_warps, int lane, Put put) {
-  for (long long r0 = warp0 * kWarp; r0 < n_rows; r0 += n_warps * kWarp) {
-    const long long r = r0 + lane;
-    const int s = r < n_rows ? order[r] : -1;
-    if (s >= n_slots) raise_status(LEWI_STATUS_BAD_INDEX);
-    const bool left = r < n_rows && s < n_slots && (s < 0 || r >= n_slot_rows || pos[s] != r);
-    for (unsigned m = __ballot_sync(0xffffffffu, left); m != 0; m &= m - 1) {
-      const int from = __ffs(m) - 1;
-      put(r0 + from, __shfl_sync(0xffffffffu, s, from));
-    }
+__device__ __forceinline__ void put_left_over(unsigned left, long long r0, int s, Put put) {
+  for (; left != 0; left &= left - 1) {
+    const int from = __ffs(left) - 1;
+    put(r0 + from, __shfl_sync(0xffffffffu, s, from));
   }
 }
 // The row of this lane's slot, -1 where nothing is to be written for it.  Without `order` pos is a permutation: a slot without a row is an error.
@@ -164,7 +164,12 @@ __device__ __forceinline__ int row_of_slot(const int32_t* __restrict__ order, in
   return in && (order == nullptr || order[p] == slot) ? p : -1;
 }
 
-// out[r] = x[order[r] / k], in token order: every row of x is read once.
+// out[r] = x[order[r] / k], in token order: every row of x is read once.  Between events, this | the row gather, in us: 16,384 tokens, k = 12,
+// d = 2048, bf16 152 | 248; 5000 tokens, k = 6, d = 1024, float32 31 | 39.  (Looking for rows left over after the tokens: 155 and 35.)
+// A warp writes the k rows of its token one after the other, so with few tokens the gather, a warp per row, is the faster one: d = 2048,
+// bf16, k = 12: 60 tokens 12 | 8, 1200 20.5 | 18.4, 2400 28.7 | 34.8; d = 1024, float32, k = 6: 60 tokens 10 | 8, 1200 14.4 | 14.2, 2400
+// 18.5 | 20.5.  The line lies at kDispatchWarps tokens per SM.
+constexpr int kDispatchWarps = 10;
 template <typename T, int VPL>
 __global__ void __launch_bounds__(kGatherThreads) dispatch_tokens_kernel(const T* __restrict__ x, const int32_t* __restrict__ order,
                                                                          const int32_t* __restrict__ pos, T* __restrict__ out,
@@ -173,8 +178,14 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_tokens_kernel(const T
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5, rows = n_tokens * k;
   const int nvec = d / Elem<T>::kPerVec;
+  auto put = [&](long long r, int s) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)(s < 0 ? 0 : s / k) * d);
+#pragma unroll 1
+    for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + r * d) + vi, s < 0 ? make_uint4(0, 0, 0, 0) : ld_nc_v4(src + vi));
+  };
+  // (k <= 32: there are no more looks of 32 rows than tokens, so a warp has one beside each of its tokens and the loads of both in flight)
   for (long long t = warp0; t < n_tokens; t += n_warps) {
-    const int my_row = lane < k ? row_of_slot(order, pos[t * k + lane], t * k + lane, rows) : -1;
+    const int my_pos = lane < k ? pos[t * k + lane] : -1, look = order != nullptr ? slot_of_row(order, t * kWarp + lane, rows) : -1;
     uint4 v[VPL];
 #pragma unroll
     for (int c = 0; c < VPL; ++c) {
@@ -182,6 +193,8 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_tokens_kernel(const T
       v[c] = make_uint4(0, 0, 0, 0);
       if (vi < nvec) v[c] = ld_nc_v4(reinterpret_cast<const uint4*>(x + t * d) + vi);
     }
+    const int my_row = lane < k ? row_of_slot(order, my_pos, t * k + lane, rows) : -1;
+    const unsigned left = order != nullptr ? left_over(pos, look, t * kWarp + lane, rows, rows, rows) : 0u;
     for (int j = 0; j < k; ++j) {
       const long long p = __shfl_sync(0xffffffffu, my_row, j);
       if (p < 0) continue;
@@ -191,13 +204,8 @@ __global__ void __launch_bounds__(kGatherThreads) dispatch_tokens_kernel(const T
         if (vi < nvec) st_v4(reinterpret_cast<uint4*>(out + p * d) + vi, v[c]);
       }
     }
+    put_left_over(left, t * kWarp, look, put);
   }
-  if (order == nullptr) return;
-  rows_left_over(order, pos, rows, rows, rows, warp0, n_warps, lane, [&](long long r, int s) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)(s < 0 ? 0 : s / k) * d);
-#pragma unroll 1
-    for (int vi = lane; vi < nvec; vi += kWarp) st_v4(reinterpret_cast<uint4*>(out + r * d) + vi, s < 0 ? make_uint4(0, 0, 0, 0) : ld_nc_v4(src + vi));
-  });
 }
 
 // out[t] = sum_j w[t,j] * y[pos[t,j]] (+ add0[t] + add1[t]); f32 accumulate.
@@ -422,6 +430,8 @@ inline int gather_grid(long long rows) {
 // requests the next row of y while it works on one.
 // 5003 tokens, k = 6, d = 1024, float32: 47 us (scaled gather and dots 35 + 39); 16,384 tokens, k = 12, d = 2048, bf16: 328 us, 5.3 TB/s
 // (240 + 207 and 32 for the rounded copy of g).  A warp per row of y instead, g out of L2 k times: 55 and 472 us.
+// Rows of 8 KB (three of them in a lane's registers, up to 255 and one CTA per SM), between events, this | what it replaces: float32,
+// d = 2048, 60 tokens, k = 6 18 | 32, 5003 96 | 148, 16,384, k = 12 539 | 810; bf16, d = 4096, 8000 tokens, k = 12 309 | 513.
 template <typename T, typename TG, int VPL>
 __global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __restrict__ y, const int32_t* __restrict__ order,
                                                                      const int32_t* __restrict__ pos, const TG* __restrict__ g,
@@ -508,7 +518,7 @@ __global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __
     if (lane < k) dw[t * k + lane] = my_dot;
   }
   if (order == nullptr) return;
-  rows_left_over(order, pos, n_dy_rows, n_rows, n * k, warp0, n_warps, lane, [&](long long r, int s) {
+  auto put = [&](long long r, int s) {
     const float sc = s < 0 ? 0.f : w[s];
 #pragma unroll 1
     for (int vi = lane; vi < nvec; vi += kWarp) {
@@ -522,7 +532,11 @@ __global__ void __launch_bounds__(kGatherThreads) combine_bwd_kernel(const T* __
       }
       st_v4(reinterpret_cast<uint4*>(dy + r * d) + vi, v);
     }
-  });
+  };
+  for (long long r0 = warp0 * kWarp; r0 < n_dy_rows; r0 += n_warps * kWarp) {
+    const int look = slot_of_row(order, r0 + lane, n_dy_rows);
+    put_left_over(left_over(pos, look, r0 + lane, n_dy_rows, n_rows, n * k), r0, look, put);
+  }
 }
 
 // Padded rows of the experts that have more than one row block: row r = x[row_slot[r] / k], zeros where row_slot[r] < 0; other experts'

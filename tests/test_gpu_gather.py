@@ -184,7 +184,8 @@ def test_token_order_dispatch_and_combine_gradients_equal_the_row_gathers(cuda, 
   assert _lib.last_status() == 0
 
 
-@pytest.mark.parametrize("t,k,d,dtype", [(1, 2, 8, "bf16"), (50, 6, 264, "f32"), (700, 4, 1024, "bf16"), (40, 12, 2048, "f32"), (6000, 3, 64, "bf16")])
+@pytest.mark.parametrize("t,k,d,dtype", [(1, 2, 8, "bf16"), (50, 6, 264, "f32"), (700, 4, 1024, "bf16"), (40, 12, 2048, "f32"), (6000, 3, 64, "bf16"),
+                                       (1479, 2, 264, "f32"), (1480, 32, 264, "f32"), (2000, 6, 1032, "bf16")])
 @pytest.mark.parametrize("tables", ["dropped", "order_only", "pos_only", "unrelated", "short"])
 def test_dispatch_and_combine_with_tables_that_are_no_permutations(cuda, t, k, d, dtype, tables):
   """Slots that were dropped (both tables negative, or one of them), tables that do not belong together, rows left out of order: every row is
