@@ -799,13 +799,10 @@ inline bool rows_map(CUtensorMap* m, const void* ptr, int cols, long long rows, 
 }
 // a [B,S,H,W] bf16 tensor: boxes of 64 tokens x 64 columns of one head; tokens and columns past the end are zero
 inline bool heads_map(CUtensorMap* m, const void* ptr, int B, int S, int H, int W) {
-  gg::EncodeTiledFn fn = gg::encode_fn();
-  if (fn == nullptr) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   const cuuint64_t strides[3] = {(cuuint64_t)W * 2, (cuuint64_t)W * H * 2, (cuuint64_t)W * H * S * 2};
-  const cuuint32_t box[4] = {64, 1, 64, 1}, estr[4] = {1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  const cuuint32_t box[4] = {64, 1, 64, 1};
+  return gg::encode_tiled(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, ptr, dims, strides, box);
 }
 
 template <int KB>

@@ -1016,35 +1016,45 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 inline EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const EncodeTiledFn fn = [] {   // (host threads that come here at the same time wait for the first)
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
+}
+
+// Tiles of 128-byte swizzled rows.  The encoder is a driver function and wants the device's context in the calling host thread, which a
+// thread has only after its first runtime call that needs one (an autograd thread whose first work is a product has none yet).
+inline bool encode_tiled(CUtensorMap* m, CUtensorMapDataType type, cuuint32_t rank, const void* ptr, const cuuint64_t* dims,
+                         const cuuint64_t* strides, const cuuint32_t* box) {
+  const EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  auto encode = [&] {
+    return fn(m, type, rank, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return false;
+    r = encode();
+  }
+  return r == CUDA_SUCCESS;
 }
 
 // bf16 (or f32) tensor [d2][d1][d0] (d0 contiguous); box [b2][b1][b0]; rank 2 when d2 == 0.
 inline bool make_map(CUtensorMap* m, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint32_t b0,
                      uint32_t b1, uint32_t b2 = 1, bool f32 = false) {
-  EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr || d0 == 0 || d1 == 0) return false;
+  if (d0 == 0 || d1 == 0) return false;
   const uint64_t esz = f32 ? 4 : 2;
   cuuint64_t dims[3] = {d0, d1, d2 ? d2 : 1};
   cuuint64_t strides[2] = {d0 * esz, d0 * d1 * esz};
   cuuint32_t box[3] = {b0, b1, b2};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const cuuint32_t rank = d2 ? 3 : 2;
-  CUresult r = fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank,
-                  const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return encode_tiled(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d2 ? 3 : 2, ptr, dims, strides, box);
 }
 
 // Tensor map of an epilogue output [d2][rows][cols]: boxes of 32 rows x 128 bytes (64 bf16 or 32 f32 columns).
