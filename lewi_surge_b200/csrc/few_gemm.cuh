@@ -4,7 +4,7 @@
 // columns are the M of the MMA (MN-major, as they lie in memory) and a block's rows its N, as many as the block has, rounded up to 16.
 // A contraction step then brings 16 KB of weights and 128 bytes per row, where the 256 x 256 tiles of a CTA pair bring 16 KB of rows
 // (mostly padding) for 16 KB of weights, and the whole ring of every SM is weights in flight.  Padding rows are neither read nor
-// computed nor stored, and the rows of the gate/up projection are picked from x by TMA gather, so no dispatch pass runs before it.
+// computed nor stored, and the rows of the gate/up projection are picked from x with cp.async, so no dispatch pass runs before it.
 // Each sum runs over the same 16-deep steps in the same order as in the pair kernels: same bits.
 //
 // warp 0 weights (TMA); warp 1 MMA; warps 2, 3, 8 and 9 rows (TMA, or cp.async where they are picked); warps 4-7 epilogue: thread =

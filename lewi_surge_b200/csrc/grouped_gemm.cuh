@@ -576,7 +576,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
 
       // DSWIGLU: this warp's 32 rows x 128 columns of g and u arrive, and dg and du leave, as TMA tiles of 32 rows x
       // 64 columns in the warp's two staging tiles: [g tile | u tile], results written in place.
-      // Lane 0 issues the copies; the first pair of loads is in flight before the accumulator is waited for.
+      // One lane issues the copies; the first pair of loads is in flight before the accumulator is waited for.
       [[maybe_unused]] const uint32_t tile_g = ptx::smem_u32(stage), tile_u = tile_g + TILE_BYTES;
       [[maybe_unused]] auto dsw_load = [&](int n) {
         if (ptx::elect_one()) {

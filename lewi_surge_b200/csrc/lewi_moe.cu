@@ -1577,8 +1577,7 @@ int lewi_moe_fwd(void* stream, void* side_stream, const void* x, const float* w_
   }
   moe::mark("router_logits", stream);
   // Few rows: from the router on each kernel starts while the one before it ends.  (Not with a mark callback, which may put events between
-  // them, and not where the side stream waits for the routing.)One decode step,
-  // launches apart and so: 8 tokens over 128 x 512 experts 68.9 -> 63.4 us, 64 tokens over 256 x 768 381 -> 371.
+  // them, and not where the side stream waits for the routing.)  One decode step, launches apart and so: 8 tokens over 128 x 512 experts 68.9 -> 63.4 us, 64 tokens over 256 x 768 381 -> 371.
   const bool early = few && !heavy && tensor_router && few_router(T, E) && moe::mark_fn() == nullptr;
   {
   moe::Range nvtx_sort("moe_permute_sort");

@@ -66,8 +66,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // True in one lane (always the same one) of a converged warp.  TMA copies and tcgen05 instructions that one thread issues stand under
 // it and not under `lane == 0`: the compiler then knows that a single thread is active.  An instruction under `lane == 0` took about
-// 100 cycles to issue (the same copies issued from one, two and four warps).  196,608 rows over 128 x 512 experts, d = 1024, under the
-// power cap: gate/up 371 -> 351 us, dx 387 -> 318, its weight gradients 371 -> 318; whole layer cases 2 to 7 %.
+// 100 cycles to issue (the same copies issued from one, two and four warps).  196,608 rows over 128 x 512 experts, d = 1024, both builds in
+// turn: gate/up 360 -> 325 us, dx and down projection 380 -> 330 and 220 -> 210; whole layer cases 2 to 7 %.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));

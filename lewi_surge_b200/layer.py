@@ -6,7 +6,7 @@ modal/padded_gmm.py:45-69) and their gather-only gradients (modal/moe_permute.py
 
   logits  = x . W_r                                   router GEMM (f32-exact on the tensor cores)
   tables  = softmax/top-k/renorm + stable sort        lewi_router_topk
-  xs      = rows of x in padded-block order           lewi_gather_rows      (dispatch)
+  xs      = rows of x in padded-block order           lewi_dispatch_rows    (dispatch; few tokens: picked by the gate/up GEMM)
   gu, h   = SwiGLU(xs . Wg[e], xs . Wu[e]) * w        gate/up GEMM, router weight folded into h
   ys      = h . Wd[e]                                 down GEMM
   shared expert on all tokens (same kernels, one group; optional sigmoid gate)
