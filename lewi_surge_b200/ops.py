@@ -40,6 +40,10 @@ def _i32(t):
   return t if t.dtype == torch.int32 else t.to(torch.int32)
 
 
+def _table(t):
+  return t if t is None or (t.dtype == torch.int32 and t.is_contiguous()) else t.to(torch.int32).contiguous()
+
+
 def padded_rows_bound(m, num_experts, block=BLOCK):
   return int(_lib.load().lewi_padded_rows_bound(int(m), int(num_experts), int(block)))
 
@@ -137,8 +141,7 @@ def dispatch_tokens(x, pos, k, order=None):
   """``gather_rows(x, order, idx_div=k)``, reading every row once where pos (N*k) is the inverse of order; without order pos is a
   permutation of the N*k rows and out[pos[t*k+j]] = x[t]."""
   lib = _lib.load()
-  x, pos = x.contiguous(), _i32(pos).contiguous()
-  order = None if order is None else _i32(order).contiguous()
+  x, pos, order = x.contiguous(), _table(pos), _table(order)
   t, d = x.shape
   out = torch.empty((t * k, d), dtype=x.dtype, device=x.device)
   check(lib.lewi_dispatch_tokens(stream(), ptr(x), ptr(order), ptr(pos), ptr(out), t, k, d, _dt(x)), "lewi_dispatch_tokens")
@@ -149,16 +152,16 @@ def combine_bwd(y, pos, g, w, order=None):
   """(dy, dw f32) of ``combine``: dy[r] = w_flat[order[r]] * g[order[r] // k], zeros where order[r] < 0, and dw[t,j] = <g[t], y[pos[t,j]]>, 0
   where pos[t,j] < 0; g rounded to y.dtype.  Without order pos is a permutation of the N*k rows and order its inverse."""
   lib = _lib.load()
-  y, pos, w = y.contiguous(), _i32(pos).contiguous(), w.to(torch.float32).contiguous()
-  g = g.contiguous()
+  y, pos, order, g = y.contiguous(), _table(pos), _table(order), g.contiguous()
+  if w.dtype != torch.float32 or not w.is_contiguous():
+    w = w.to(torch.float32).contiguous()
   if g.dtype != y.dtype and (g.dtype != torch.float32 or g.data_ptr() % 16):   # (the kernel rounds float32 rows that start on 16 bytes)
     g = g.to(y.dtype)
   (n, k), d = w.shape, y.shape[1]
-  order = None if order is None else _i32(order).contiguous()
   if pos.numel() != n * k or g.shape != (n, d) or (order is None and y.shape[0] != n * k):
     raise LewiError("combine_bwd: y (N*k, D), pos (N, k), g (N, D), w (N, k)")
   rows = n * k if order is None else order.shape[0]
-  dy, dw = torch.empty((rows, d), dtype=y.dtype, device=y.device), torch.empty_like(w)
+  dy, dw = torch.empty_like(y) if rows == y.shape[0] else y.new_empty((rows, d)), torch.empty_like(w)
   if n * k > 0:
     check(lib.lewi_combine_bwd(stream(), ptr(y), ptr(order), ptr(pos), ptr(g), ptr(w), ptr(dy), ptr(dw), n, k, d, y.shape[0], rows, _dt(y),
                                _dt(g)), "lewi_combine_bwd")
